@@ -739,9 +739,38 @@ bool check_shape(IncNtt* t, const uint32_t* limbs, uint32_t L, uint32_t special,
 // Forward transforms of every digit: D[b][j][i] = NTT(d_j mod q_i), reading digit
 // rows from src (limb j at src + j N, polynomials src_stride apart).
 // skip_diag: the rows i == j are already in D (k_tensor's dd) and are not transformed.
+//
+// FP64 primes take one transform for all nd digits.  One transform per digit has too few
+// rows to fill the GPU when the batch is small, and each of its launches ends in a partly
+// empty wave.  Measured on B200 against one transform per digit: 78 -> 51 us for one
+// multiply at N = 2^13, L = 4; 268 -> 193 us for 8 rotations at 2^14, L = 9; 1790 -> 1560
+// us for 3 at 2^16, L = 24; unchanged for 256 multiplies at 2^14, L = 9.  Groups of
+// digits sized to stay in L2 between the column and the tile pass were slower than one
+// group at every size tried (32 to 1000 MB), so there is no such limit.
 int digits_forward(IncNtt* t, uint64_t* D, const uint64_t* src, long long src_stride, uint64_t B,
                    const uint32_t* ext, int nd, int ne, cudaStream_t st, bool skip_diag = false) {
     const long long N = (long long)t->pub.N;
+    RowSet all;
+    memset(&all, 0, sizeof all);
+    for (int i = 0; i < ne; ++i) {
+        all.in[i] = src;
+        all.out[i] = D + (long long)i * N;
+        all.prime[i] = ext[i];
+    }
+    all.nlimbs = ne;
+    mark_fp64(all, t);  // looks at all ne primes
+    all.nlimbs = skip_diag ? ne - 1 : ne;
+    all.split = (int)t->pub.split_degree;
+    all.logP = t->logP;
+    all.batch = (int)B;
+    all.batch_stride = (long long)nd * ne * N;
+    all.in_batch_stride = src_stride;
+    all.reduce_input = 1;
+    all.digits = nd;
+    all.skip_diag = skip_diag ? 1 : 0;
+    all.digit_in_stride = N;
+    all.digit_stride = (long long)ne * N;
+    if (ntt_f64_eligible(all)) return launch_ntt(all, t->d_info, false, st);
     for (int j = 0; j < nd; ++j) {
         RowSet rs;
         memset(&rs, 0, sizeof rs);

@@ -132,8 +132,8 @@ int launch_ntt_f64(const RowSet& rows, const PrimeInfo* d_primes, bool inverse, 
 namespace {
 // The register-blocked kernels use 16-byte vector accesses on row segments.
 bool rows_aligned16(const RowSet& rows) {
-    if ((rows.batch_stride | rows.in_batch_stride) & 1) return false;
-    for (int k = 0; k < rows.nlimbs; ++k)
+    if ((rows.batch_stride | rows.in_batch_stride | rows.digit_stride | rows.digit_in_stride) & 1) return false;
+    for (int k = 0; k < rowset_slots(rows); ++k)
         if ((((uintptr_t)rows.out[k]) | ((uintptr_t)rows.in[k])) & 15) return false;
     return true;
 }
@@ -169,6 +169,7 @@ int launch_ntt(const RowSet& rows, const PrimeInfo* d_primes, bool inverse, cuda
         return e == -1 ? (int)cudaErrorInvalidValue : e;
     }
     if (rows.batch <= 0 || rows.nlimbs <= 0) return 0;
+    if (rows.digits && !ntt_f64_eligible(rows)) return (int)cudaErrorInvalidValue;  // FP64 path only
     read_force_flags();
     if (!g_force_generic && logP >= 8 && logP <= 17 && rows_aligned16(rows)) {
         if (rows.fp64 && !g_force_int) {

@@ -60,12 +60,25 @@ struct RowSet {
     const RowDesc* table;
     long long table_rows;
     int table_src_is_dst;  // read table[r].out instead of .in (second pass of a split transform)
+    // Digit mode (FP64 path only): when `digits` is set, polynomial b is `digits` digit
+    // polynomials, each transformed modulo every limb slot, and digit j of polynomial b,
+    // slot k, is row ((b * digits + j) * nlimbs + k):
+    //   in  = in_base[k]  + b * in_batch_stride + j * digit_in_stride
+    //   out = out_base[k] + b * batch_stride    + j * digit_stride
+    // With skip_diag, digit j leaves out slot j: nlimbs counts the slots left and the
+    // arrays hold nlimbs + 1.
+    int digits, skip_diag;
+    long long digit_in_stride, digit_stride;
 };
 
 // Rows one launch of `rows` transforms.
 inline long long rowset_rows(const RowSet& rows) {
-    return rows.table ? rows.table_rows : (long long)rows.batch * rows.nlimbs * rows.split;
+    return rows.table ? rows.table_rows
+                      : (long long)rows.batch * rows.nlimbs * rows.split * (rows.digits ? rows.digits : 1);
 }
+
+// Entries of a row set's slot arrays.
+inline int rowset_slots(const RowSet& rows) { return rows.nlimbs + (rows.digits && rows.skip_diag ? 1 : 0); }
 
 // Launch shape of the FP64 transform for one (log2 P, log2 rows) class:
 //   tile_bits      low index bits done by one CTA tile (== logP: one pass; else a

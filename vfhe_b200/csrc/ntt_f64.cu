@@ -633,8 +633,9 @@ int launch_ntt_f64(const RowSet& rows, const PrimeInfo* d_primes, bool inverse, 
     if (sc.ctas_per_sm == -1 && K >= 11 && K <= 13 && K1 >= 1 && K1 <= 3)
         return fused_dispatch(K, K1, rows, d_primes, inverse, stream);
     RowSet second = rows;
-    for (int i = 0; i < rows.nlimbs; ++i) second.in[i] = rows.out[i];
+    for (int i = 0; i < rowset_slots(rows); ++i) second.in[i] = rows.out[i];
     second.in_batch_stride = rows.batch_stride;
+    second.digit_in_stride = rows.digit_stride;
     second.reduce_input = 0;
     second.table_src_is_dst = 1;
     int e;

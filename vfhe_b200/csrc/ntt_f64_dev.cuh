@@ -249,6 +249,35 @@ struct Tile {
     int hi;
 };
 
+// Where row `row` of a launch starts (slot-addressed rows): input, output and prime.
+struct RowAt {
+    const uint64_t* src;
+    uint64_t* dst;
+    uint32_t prime;
+};
+
+__device__ __forceinline__ RowAt row_at(const RowSet& rows, long long row) {
+    const int per_poly = rows.nlimbs * rows.split;
+    long long b = row / per_poly;
+    const int rem = (int)(row - b * per_poly);
+    int slot = rem / rows.split;
+    const int blk = rem - slot * rows.split;
+    long long in_off = (long long)blk << rows.logP, out_off = in_off;
+    if (rows.digits) {
+        const long long bj = b;
+        b = bj / rows.digits;
+        const int j = (int)(bj - b * rows.digits);
+        if (rows.skip_diag && slot >= j) ++slot;
+        in_off += j * rows.digit_in_stride;
+        out_off += j * rows.digit_stride;
+    }
+    RowAt r;
+    r.src = rows.in[slot] + b * rows.in_batch_stride + in_off;
+    r.dst = rows.out[slot] + b * rows.batch_stride + out_off;
+    r.prime = rows.prime[slot];
+    return r;
+}
+
 template <bool TABLE>
 __device__ __forceinline__ Tile locate(const RowSet& rows, const PrimeInfo* primes, int K, long long tile,
                                        int tiles_per_row) {
@@ -264,15 +293,11 @@ __device__ __forceinline__ Tile locate(const RowSet& rows, const PrimeInfo* prim
         r.pi = d.pi;
         return r;
     }
-    const int per_poly = rows.nlimbs * rows.split;
-    const long long b = row / per_poly;
-    const int rem = (int)(row - b * per_poly);
-    const int slot = rem / rows.split;
-    const int blk = rem - slot * rows.split;
-    const long long off = ((long long)blk << rows.logP) + ((long long)hi << K);
-    r.src = rows.in[slot] + b * rows.in_batch_stride + off;
-    r.dst = rows.out[slot] + b * rows.batch_stride + off;
-    r.pi = primes + rows.prime[slot];
+    const RowAt at = row_at(rows, row);
+    const long long off = (long long)hi << K;
+    r.src = at.src + off;
+    r.dst = at.dst + off;
+    r.pi = primes + at.prime;
     return r;
 }
 
@@ -521,15 +546,10 @@ __device__ __forceinline__ void col_one(const RowSet& rows, const PrimeInfo* __r
         dst = d.out + cc;
         pp = d.pi;
     } else {
-        const int per_poly = rows.nlimbs * rows.split;
-        const long long b = row / per_poly;
-        const int rem = (int)(row - b * per_poly);
-        const int slot = rem / rows.split;
-        const int blk = rem - slot * rows.split;
-        const long long off = ((long long)blk << rows.logP) + cc;
-        src = rows.in[slot] + b * rows.in_batch_stride + off;
-        dst = rows.out[slot] + b * rows.batch_stride + off;
-        pp = primes + rows.prime[slot];
+        const RowAt at = row_at(rows, row);
+        src = at.src + cc;
+        dst = at.dst + cc;
+        pp = primes + at.prime;
     }
     const PrimeInfo& pi = *pp;
     const double q = pi.qd, qinv = pi.qinv;
