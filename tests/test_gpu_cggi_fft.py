@@ -146,3 +146,49 @@ def test_keyswitch_mismatches_come_from_key_noise(cuda, torus_oracle):
         exact_ext = oracle_bootstrap(torus_oracle, lwe_i[None], tv, keys.bsk, p)
         assert keys.decrypt(exact_ext, keys.S)[0] == keys.decrypt(ext_i[None], keys.S)[0] == lut[m_i]
         assert np.array_equal(oracle_keyswitch(torus_oracle, ext_i[None], keys.ksk, p)[0], out_i)
+
+
+@pytest.mark.parametrize("N,levels,base_log", [(512, 1, 7), (512, 3, 7), (1024, 2, 8), (1024, 3, 7), (1024, 4, 6),
+                                               (2048, 3, 7)])
+def test_blind_rotation_is_exact_on_both_block_shapes(cuda, torus_oracle, N, levels, base_log):
+    """A few LWEs run on wide blocks (N <= 1024), more than one per SM on two-group blocks.
+    The external products' sums stay below 2^51 here and the transforms' error far below one
+    half, so every coefficient rounds to the exact product: both equal the integer oracle."""
+    import torch
+
+    from vfhe_b200.cggi_fft import CggiFft, TorusKeys, TorusParams, to_device, to_host
+
+    p = TorusParams(n=5, N=N, bs_levels=levels, bs_base_log=base_log)
+    rng = np.random.default_rng(N + levels)
+    keys = TorusKeys.generate(p, rng)
+    dev = CggiFft(keys, cuda)
+    tv = rng.integers(0, 1 << 32, N, dtype=np.uint64).astype(np.uint32)
+    many = torch.cuda.get_device_properties(0).multi_processor_count + 3
+    lwe = rng.integers(0, 1 << 32, (many, p.n + 1), dtype=np.uint64).astype(np.uint32)
+    few = to_host(dev.blind_rotate(to_device(lwe[:3]), to_device(tv)))
+    all_ = to_host(dev.blind_rotate(to_device(lwe), to_device(tv)))
+    want = oracle_bootstrap(torus_oracle, lwe[:3], tv, keys.bsk, p)
+    assert np.array_equal(few, want)
+    assert np.array_equal(all_[:3], want)
+    assert np.array_equal(all_[-2:], oracle_bootstrap(torus_oracle, lwe[-2:], tv, keys.bsk, p))
+
+
+@pytest.mark.parametrize("n,N,base_log,levels,batch", [(1, 1, 1, 1, 1), (31, 33, 2, 8, 32), (32, 64, 4, 3, 33),
+                                                       (630, 1024, 2, 8, 7), (63, 70, 8, 4, 129), (95, 40, 1, 16, 16)])
+def test_keyswitch_tiles_and_shares(cuda, torus_oracle, n, N, base_log, levels, batch):
+    """Edges of the tensor tiles (ciphertexts, columns, digits) and mask shares, bit for bit."""
+    import torch
+
+    from vfhe_b200.cggi_fft import TorusParams, to_device, to_host
+
+    p = TorusParams(n=n, N=N, ks_base_log=base_log, ks_levels=levels)
+    rng = np.random.default_rng(n + N)
+    ksk = rng.integers(0, 1 << 32, (N, levels, n + 1), dtype=np.uint64).astype(np.uint32)
+    ext = rng.integers(0, 1 << 32, (batch, N + 1), dtype=np.uint64).astype(np.uint32)
+    d_in, d_k = to_device(ext), to_device(ksk)
+    out = torch.full((batch, n + 1), -1, dtype=torch.int32, device="cuda")
+    u32 = lambda t: cuda.ffi.cast("uint32_t*", t.data_ptr())  # noqa: E731
+    assert cuda.lib.vfhe_cuda_cggi_fft_keyswitch_batch(
+        u32(out), u32(d_in), batch, u32(d_k), N, n, base_log, levels,
+        cuda.ffi.cast("void*", torch.cuda.current_stream().cuda_stream)) == 0
+    assert np.array_equal(to_host(out), oracle_keyswitch(torus_oracle, ext, ksk, p))
