@@ -68,3 +68,52 @@ def test_batched_bootstrap_matches_reference_path(cuda, N, n_lwe, count):
         o.set_rows(to_host(oa)[i], to_host(ob)[i])
         ph = o.phase(key2, recompose=True)
         assert round(ph * (2 * t) / in_ring.q_l) % (2 * t) == lut[m]
+
+
+@pytest.mark.parametrize("N,L0", [(256, 1), (256, 2), (512, 1), (512, 2), (1024, 1), (1024, 2), (2048, 2), (4096, 1)])
+def test_fused_forms_match_one_launch_per_stage(cuda, N, L0):
+    """A key off the 16-byte boundary takes one launch per stage.  The same key on it takes
+    whole rotations on clusters for a few LWEs (N <= 2048) and one launch per step for many
+    (512 <= N): the same residues from uniform keys, ciphertexts and test vectors."""
+    import torch
+
+    from vfhe_b200.arith import Ring
+
+    n, few, many, t = 9, 3, 150, 16
+    R = Ring(N, prime_size=[50] * (L0 + 1), split_degree=1, engine=cuda)
+    q, limbs = R.primes, cuda.ffi.new("uint32_t[]", R.prime_indices[:L0])
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(N + L0)
+
+    def uniform(shape, axis, primes):
+        x = torch.empty(shape, dtype=torch.int64, device="cuda")
+        for k, p in enumerate(primes):
+            x.select(axis, k).random_(0, p, generator=gen)
+        return x
+
+    a, b = uniform((many, L0, n), 1, q[:L0]), uniform((many, L0), 1, q[:L0])
+    a[1] = 0  # rotations by zero
+    bk, tv = uniform((n, 2 * L0, 2, L0 + 1, N), 3, q), uniform((2, L0, N), 1, q[:L0])
+    off = torch.empty(bk.numel() + 1, dtype=torch.int64, device="cuda")
+    off[1:] = bk.flatten()
+
+    def run(count, key_ptr):
+        oa = torch.empty((count, L0, N), dtype=torch.int64, device="cuda")
+        ob = torch.empty((count, L0), dtype=torch.int64, device="cuda")
+        ws = torch.empty(cuda.lib.vfhe_cuda_cggi_workspace_bytes(R.NTT, count, n, L0) // 8 + 1, dtype=torch.int64,
+                         device="cuda")
+        p = lambda x: cuda.ffi.cast("uint64_t*", x.data_ptr())  # noqa: E731
+        rc = cuda.lib.vfhe_cuda_cggi_bootstrap_batch(
+            R.NTT, p(oa), p(ob), p(a), p(b), count, n, limbs, L0, R.prime_indices[L0],
+            cuda.ffi.cast("uint64_t*", key_ptr), p(tv), t, cuda.ffi.cast("void*", ws.data_ptr()),
+            cuda.ffi.cast("void*", torch.cuda.current_stream().cuda_stream))
+        cuda.check("bootstrap")
+        assert rc == 0
+        torch.cuda.synchronize()
+        return oa, ob
+
+    assert bk.data_ptr() % 16 == 0 and off.data_ptr() % 16 == 0
+    want_a, want_b = run(many, off.data_ptr() + 8)
+    for count in (few, many):
+        oa, ob = run(count, bk.data_ptr())
+        assert torch.equal(oa, want_a[:count]) and torch.equal(ob, want_b[:count])

@@ -11,11 +11,15 @@
 // ExtProd: digit d = limb l of component c of the difference, lifted to the key's
 // extended limbs and transformed; accumulated against bk_i[d]; inverse transform;
 // rounded division by the special prime.
+// Three forms with the same residues: whole rotations on clusters (small batches), one
+// launch per step for the external product and one for the division (k_cggi_step), and one
+// launch per stage (rings or keys the fused kernels do not take).
 //
 // The accumulator stays in the coefficient domain: the reference transforms the CMUX
 // output forward (mgsw.c:48,67) and the next step back (cggi16.py:84); both maps are
 // exact inverses on canonical residues, so skipping them leaves every bit unchanged.
 // A step with a_i' = 0 (skipped by the reference) adds ExtProd(bk_i, 0) = 0 here.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <string.h>
 
@@ -23,6 +27,7 @@
 
 #include "abi_common.cuh"
 #include "fp64mod.cuh"
+#include "ntt_f64_dev.cuh"
 
 namespace vc {
 
@@ -244,6 +249,498 @@ __global__ void k_moddown_acc(uint64_t* __restrict__ acc, const uint64_t* __rest
     }
 }
 
+__device__ __forceinline__ void group_sync(int grp, int threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(threads) : "memory");
+}
+
+// ---- whole blind rotations on a cluster
+//
+// One cluster of L0 + 1 blocks runs one LWE's n CMUX steps, block e for extended prime e.
+// Group d of N / 8 threads keeps limb d % L0 of component d / L0 of the accumulator in
+// registers (every block a copy), forms digit d of acc X^r - acc, transforms it modulo the
+// block's prime; the block multiplies the digits with its limb of the key and transforms the
+// two outputs back.  The outputs go through L2 to the other blocks, which divide by the
+// special prime and add: one cluster barrier a step.
+//
+// For batches of up to one block per SM, where a step's latency counts.  The transforms hold
+// 8 residues a thread (three stages a pass) instead of the 16 of the tile kernels, so that a
+// block has twice the warps.
+//
+// N = 1024, L0 = 2, n = 630: 18 us a step with five launches, 8.5 us here (about 4000 cycles
+// forward, 1300 products, 4000 inverse, the rest barriers and the exchange through L2).
+
+__device__ __forceinline__ int pad8(int i) { return i + ((i >> 4) << 1); }
+
+// Pass P of a 2^K-point transform in 8-residue passes: three index bits from the top, the
+// last pass the K mod 3 bits left (none: K / 3 passes).  index() is residue k's place for
+// thread t; a partial pass takes its low bits and the index's top bits, so that the lanes
+// of a warp own consecutive groups.
+template <int K, int P>
+struct Pass8 {
+    static constexpr int FULL = K / 3;
+    static constexpr bool PARTIAL = P >= FULL;
+    static constexpr int LO = PARTIAL ? 0 : K - 3 * (P + 1);
+    static constexpr int NST = PARTIAL ? K % 3 : 3;
+    __device__ __forceinline__ static int index(int t, int k) {
+        if constexpr (PARTIAL) {
+            return ((k >> NST) << (K - 3 + NST)) | (t << NST) | (k & ((1 << NST) - 1));
+        } else {
+            return ((t >> LO) << (LO + 3)) | (k << LO) | (t & ((1 << LO) - 1));
+        }
+    }
+    // The butterflies at field bit bb have 2^(2-bb) twiddles (partial pass: 8 / 2^(bb+1)), by
+    // k >> (bb + 1); stage bb's start at offset(bb).
+    static constexpr int offset(int bb) { return bb == 0 ? 0 : bb == 1 ? 4 : 6; }
+};
+
+// The pass's twiddles, requested before the exchange that precedes it so that their latency
+// overlaps the barrier (tables by 2^(K-1-b) + (i >> (b + 1)) for index bit b).
+struct Twiddles8 {
+    double2 w[7];
+};
+
+template <int K, int P>
+__device__ __forceinline__ void load_twiddles(Twiddles8& T, const double2* tw, int t) {
+    using Q = Pass8<K, P>;
+#pragma unroll
+    for (int bb = 0; bb < Q::NST; ++bb) {
+        const int b = Q::LO + bb;
+#pragma unroll
+        for (int h = 0; h < (4 >> bb); ++h)
+            T.w[Q::offset(bb) + h] = __ldg(&tw[(1 << (K - 1 - b)) + (Q::index(t, h << (bb + 1)) >> (b + 1))]);
+    }
+}
+
+template <int K>
+struct Passes8 {
+    static constexpr int count = (K + 2) / 3;
+};
+
+template <int K, int P>
+__device__ __forceinline__ void put_regs(double* sm, const double (&x)[8], int t) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) sm[pad8(Pass8<K, P>::index(t, k))] = x[k];
+}
+
+template <int K, int P>
+__device__ __forceinline__ void get_regs(double (&x)[8], const double* sm, int t) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) x[k] = sm[pad8(Pass8<K, P>::index(t, k))];
+}
+
+// Forward (Cooley-Tukey) passes P.. of 8 residues a thread in pass P's layout; every fourth
+// stage of the transform ends with a reduction (|x| <= q in, each stage adds at most 3q/4,
+// so every product's operand stays below 4q < 2^52).  Out: the last pass's layout, |x| < 4q.
+template <int K, int P>
+__device__ __forceinline__ void fwd8(double (&x)[8], const Twiddles8& T, double* sm, int t, int grp, const double2* tw,
+                                     double q, double qinv) {
+    using Q = Pass8<K, P>;
+#pragma unroll
+    for (int bb = Q::NST - 1; bb >= 0; --bb) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if (k & (1 << bb)) continue;
+            const double2 w = T.w[Q::offset(bb) + (k >> (bb + 1))];
+            const double v = f_mulmod(x[k | (1 << bb)], w.x, w.y, q);
+            const double u = x[k];
+            x[k] = __dadd_rn(u, v);
+            x[k | (1 << bb)] = __dsub_rn(u, v);
+        }
+        const int stage = K - (Q::LO + bb);  // stages done so far
+        if ((stage & 3) == 0 && stage != K) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) x[k] = f_reduce(x[k], q, qinv);
+        }
+    }
+    if constexpr (P + 1 < Passes8<K>::count) {
+        Twiddles8 next;
+        load_twiddles<K, P + 1>(next, tw, t);
+        group_sync(grp, 1 << (K - 3));  // the buffer's last contents are read
+        put_regs<K, P>(sm, x, t);
+        group_sync(grp, 1 << (K - 3));
+        get_regs<K, P + 1>(x, sm, t);
+        fwd8<K, P + 1>(x, next, sm, t, grp, tw, q, qinv);
+    }
+}
+
+// Inverse (Gentleman-Sande) passes P down to 0, residues in pass P's layout, |x| <= q / 2 + 1
+// in.  Sums double with every stage: three stages reach 4q < 2^52, so the sums are reduced at
+// the end of each pass.  P^-1 is folded into the last stage; |x| <= 3q/4 out, pass 0's layout.
+template <int K, int P>
+__device__ __forceinline__ void inv8(double (&x)[8], const Twiddles8& T, double* sm, int t, int grp, const PrimeInfo& pi) {
+    using Q = Pass8<K, P>;
+    const double q = pi.qd, qinv = pi.qinv;
+#pragma unroll
+    for (int bb = 0; bb < Q::NST; ++bb) {
+        const bool last = P == 0 && bb == Q::NST - 1;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if (k & (1 << bb)) continue;
+            const double u = x[k], v = x[k | (1 << bb)];
+            if (last) {
+                x[k] = f_mulmod(__dadd_rn(u, v), pi.pinv_d, pi.pinv_q, q);
+                x[k | (1 << bb)] = f_mulmod(__dsub_rn(u, v), pi.ilast_d, pi.ilast_q, q);
+            } else {
+                const double2 w = T.w[Q::offset(bb) + (k >> (bb + 1))];
+                x[k] = __dadd_rn(u, v);
+                x[k | (1 << bb)] = f_mulmod(__dsub_rn(u, v), w.x, w.y, q);
+            }
+        }
+    }
+    if constexpr (P > 0) {
+        Twiddles8 next;
+        load_twiddles<K, P - 1>(next, reinterpret_cast<const double2*>(pi.inv_d), t);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) x[k] = f_reduce(x[k], q, qinv);
+        group_sync(grp, 1 << (K - 3));
+        put_regs<K, P>(sm, x, t);
+        group_sync(grp, 1 << (K - 3));
+        get_regs<K, P - 1>(x, sm, t);
+        inv8<K, P - 1>(x, next, sm, t, grp, pi);
+    }
+}
+
+// A key pair loaded where the call stands (not moved to its use).
+__device__ __forceinline__ ulonglong2 load_key(const uint64_t* p) {
+    ulonglong2 v;
+    asm volatile("ld.global.nc.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p));
+    return v;
+}
+
+template <int K, int L0>
+struct ClusterShape {
+    static constexpr int N = 1 << K, NE = L0 + 1, ND = 2 * L0, TPT = 1 << (K - 3), THREADS = ND * TPT;
+    static constexpr int PADDED = N + (N >> 3);
+    static constexpr size_t smem = 8 * (size_t)(ND * PADDED);  // exchange buffers
+};
+
+template <int K, int L0>
+__global__ void __launch_bounds__(ClusterShape<K, L0>::THREADS)
+    k_cggi_cluster(uint64_t* __restrict__ out_a, uint64_t* __restrict__ out_b, double* ext0, double* ext1,
+                   const uint64_t* __restrict__ tv, const uint64_t* __restrict__ bk, const uint32_t* __restrict__ rots,
+                   const uint32_t* __restrict__ rot0, const __grid_constant__ CggiShape sh,
+                   const __grid_constant__ DivConsts dc, const PrimeInfo* __restrict__ primes, long long B) {
+    using C = ClusterShape<K, L0>;
+    constexpr int N = C::N, NE = C::NE, ND = C::ND, TPT = C::TPT, T = C::THREADS, PADDED = C::PADDED;
+    constexpr int NP = Passes8<K>::count;
+    extern __shared__ __align__(128) double ex[];
+    namespace cgx = cooperative_groups;
+    cgx::cluster_group cluster = cgx::this_cluster();
+    const int e = (int)cluster.block_rank();
+    const long long b = blockIdx.x / NE;
+    const int tid = threadIdx.x, g = tid / TPT, t = tid - g * TPT;
+    const PrimeInfo& pi = primes[sh.ext_prime[e]];
+    const double q = pi.qd, qinv = pi.qinv;
+    const double2* fwd = reinterpret_cast<const double2*>(pi.fwd_d);
+    double* exg = ex + g * PADDED;
+    // this LWE's outputs [2][NE][N] as doubles, in the buffer of the step's parity
+    ext0 += b * 2 * NE * N;
+    ext1 += b * 2 * NE * N;
+    // group g keeps limb dl of component dcomp of the accumulator, 8 residues a thread
+    const int dl = g % L0, dcomp = g / L0;
+    const PrimeInfo& pl = primes[sh.lwe_prime[dl]];
+    const uint64_t ql = pl.q;
+    uint64_t u[8];
+    {  // acc = tv X^rot0 (mlwe_RNSc_mul_by_xai, rns_polynomial.c:1048-1106)
+        const uint32_t a = rot0[b];
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+            const uint32_t s = ((uint32_t)Pass8<K, 0>::index(t, m) + 2 * N - a) & (2 * N - 1);
+            const uint64_t v = tv[(long long)g * N + (s & (N - 1))];
+            u[m] = s < (uint32_t)N ? v : neg_mod(v, ql);
+        }
+    }
+    uint32_t r = rots[b];
+    for (int i = 0; i < sh.n; ++i) {
+        const uint32_t r_next = i + 1 < sh.n ? __ldg(rots + (long long)(i + 1) * B + b) : 0;
+        const uint64_t* key = bk + (long long)i * (ND * 2 * NE) * N + (long long)e * N;
+        if (i + 1 < sh.n && tid < ND * 2)  // the next step's limb rows on their way to L2
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(key + (long long)(ND * 2 + tid) * NE * N),
+                         "n"(N * 8)
+                         : "memory");
+        // this step's key at the thread's multiply positions, on its way during the transforms
+        constexpr int TURNS = N / (2 * T);
+        ulonglong2 kv[TURNS][ND][2];
+#pragma unroll
+        for (int k = 0; k < TURNS; ++k)
+#pragma unroll
+            for (int d = 0; d < ND; ++d)
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+                    kv[k][d][c] = load_key(key + (long long)(2 * d + c) * NE * N + 2 * (tid + k * T));
+        // digit g of acc X^r - acc (mgsw_CMUX's in2 - in1, mgsw.c:60-61), modulo this prime;
+        // the rotated limb through the group's buffer
+        double x[8];
+        Twiddles8 tw0;
+        load_twiddles<K, 0>(tw0, fwd, t);
+        {
+            uint64_t* rowbuf = reinterpret_cast<uint64_t*>(exg);
+#pragma unroll
+            for (int m = 0; m < 8; ++m) rowbuf[Pass8<K, 0>::index(t, m)] = u[m];
+            group_sync(g, TPT);
+#pragma unroll
+            for (int m = 0; m < 8; ++m) {
+                const uint32_t s = ((uint32_t)Pass8<K, 0>::index(t, m) + 2 * N - r) & (2 * N - 1);
+                const uint64_t v = rowbuf[s & (N - 1)];
+                uint64_t d = s < (uint32_t)N ? v - u[m] : 0 - v - u[m];
+                // d is in (-2q, q) modulo 2^64
+                if ((long long)d < 0) d += ql;
+                if ((long long)d < 0) d += ql;
+                x[m] = f_from_u64(d);
+                if (dl != e) x[m] = f_reduce(x[m], q, qinv);
+            }
+        }
+        fwd8<K, 0>(x, tw0, exg, t, g, fwd, q, qinv);
+#pragma unroll
+        for (int m = 0; m < 8; ++m) x[m] = f_reduce(x[m], q, qinv);
+        group_sync(g, TPT);  // the last exchange is read
+        put_regs<K, NP - 1>(exg, x, t);
+        __syncthreads();
+        // both outputs at two positions a turn: sums of ND products, |sum| <= 3q
+        double s[TURNS][2][2];
+#pragma unroll
+        for (int k = 0; k < TURNS; ++k) {
+            const int xx = 2 * (tid + k * T);
+            s[k][0][0] = s[k][0][1] = s[k][1][0] = s[k][1][1] = 0.0;
+#pragma unroll
+            for (int d = 0; d < ND; ++d) {
+                const ulonglong2 ka = kv[k][d][0], kb = kv[k][d][1];
+                const double2 v = *reinterpret_cast<const double2*>(ex + d * PADDED + pad8(xx));
+                const double w0 = __dmul_rn(v.x, qinv), w1 = __dmul_rn(v.y, qinv);
+                s[k][0][0] = __dadd_rn(s[k][0][0], f_mulmod(f_from_u64(ka.x), v.x, w0, q));
+                s[k][0][1] = __dadd_rn(s[k][0][1], f_mulmod(f_from_u64(ka.y), v.y, w1, q));
+                s[k][1][0] = __dadd_rn(s[k][1][0], f_mulmod(f_from_u64(kb.x), v.x, w0, q));
+                s[k][1][1] = __dadd_rn(s[k][1][1], f_mulmod(f_from_u64(kb.y), v.y, w1, q));
+            }
+        }
+        __syncthreads();  // every spectrum is read
+#pragma unroll
+        for (int k = 0; k < TURNS; ++k) {
+            const int xx = 2 * (tid + k * T);
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+                *reinterpret_cast<double2*>(ex + c * PADDED + pad8(xx)) =
+                    make_double2(f_reduce(s[k][c][0], q, qinv), f_reduce(s[k][c][1], q, qinv));
+        }
+        __syncthreads();
+        double* ext = (i & 1) ? ext1 : ext0;
+        if (g < 2) {  // output g back to coefficients, for every block of the cluster
+            Twiddles8 twi;
+            load_twiddles<K, NP - 1>(twi, reinterpret_cast<const double2*>(pi.inv_d), t);
+            get_regs<K, NP - 1>(x, exg, t);
+            inv8<K, NP - 1>(x, twi, exg, t, g, pi);
+            double* o = ext + (g * NE + e) * N;
+#pragma unroll
+            for (int m = 0; m < 8; ++m) {
+                if (e == L0) {  // the special prime's: (x + p/2) mod p
+                    uint64_t v = f_to_canonical(x[m], q, qinv, pi.q) + dc.half_p;
+                    v -= v >= dc.p ? dc.p : 0;
+                    x[m] = f_from_u64(v);
+                }
+                o[Pass8<K, 0>::index(t, m)] = x[m];
+            }
+        }
+        cluster.sync();
+        // round division by the special prime (rns_polynomial.c:939-976) + in1 (mgsw.c:65-68).
+        // The other parity's buffer is written meanwhile; this one again only after the next
+        // barrier, which every block reaches past these reads.
+        {
+            const double* ev = ext + (dcomp * NE + dl) * N;
+            const double* tp = ext + (dcomp * NE + L0) * N;
+            double y[8], td[8];
+#pragma unroll
+            for (int m = 0; m < 8; ++m) {
+                y[m] = __ldcg(ev + Pass8<K, 0>::index(t, m));
+                td[m] = __ldcg(tp + Pass8<K, 0>::index(t, m));
+            }
+#pragma unroll
+            for (int m = 0; m < 8; ++m) {
+                const double z = __dadd_rn(__dadd_rn(y[m], dc.half_sp_d[dl]), -td[m]);
+                const double v = __dadd_rn(f_mulmod(z, dc.inv_sp_d[dl], dc.inv_sp_dq[dl], pl.qd), f_from_u64(u[m]));
+                u[m] = f_to_canonical(v, pl.qd, pl.qinv, ql);
+            }
+        }
+        r = r_next;
+    }
+    // sample extraction at coefficient 0 (mlwe.c:40-68)
+    if (e == 0) {
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+            const int j = Pass8<K, 0>::index(t, m);
+            if (dcomp == 0) out_a[(b * L0 + dl) * N + ((N - j) & (N - 1))] = j == 0 ? u[m] : neg_mod(u[m], ql);
+            else if (j == 0) out_b[b * L0 + dl] = u[m];
+        }
+    }
+}
+
+template <int K, int L0>
+int launch_cluster_t(uint64_t* out_a, uint64_t* out_b, double* ext0, double* ext1, const uint64_t* tv, const uint64_t* bk, const uint32_t* rots,
+                     const uint32_t* rot0, const CggiShape& sh, const DivConsts& dc, const PrimeInfo* dp, uint64_t B,
+                     cudaStream_t st) {
+    using C = ClusterShape<K, L0>;
+    int e = (int)cudaFuncSetAttribute(k_cggi_cluster<K, L0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem);
+    if (e) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(B * C::NE), 1, 1);
+    cfg.blockDim = dim3(C::THREADS, 1, 1);
+    cfg.dynamicSmemBytes = C::smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = C::NE;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e = (int)cudaLaunchKernelEx(&cfg, k_cggi_cluster<K, L0>, out_a, out_b, ext0, ext1, tv, bk, rots, rot0, sh, dc, dp, (long long)B);
+    if (e) return e;
+    note_launch();
+    return (int)cudaGetLastError();
+}
+
+// -1 for shapes without a cluster kernel.
+int launch_cluster(int K, uint64_t* out_a, uint64_t* out_b, double* ext0, double* ext1, const uint64_t* tv, const uint64_t* bk, const uint32_t* rots,
+                   const uint32_t* rot0, const CggiShape& sh, const DivConsts& dc, const PrimeInfo* dp, uint64_t B,
+                   cudaStream_t st) {
+    switch (K * 4 + sh.L0) {
+        case 8 * 4 + 1: return launch_cluster_t<8, 1>(out_a, out_b, ext0, ext1, tv, bk, rots, rot0, sh, dc, dp, B, st);
+        case 8 * 4 + 2: return launch_cluster_t<8, 2>(out_a, out_b, ext0, ext1, tv, bk, rots, rot0, sh, dc, dp, B, st);
+        case 9 * 4 + 1: return launch_cluster_t<9, 1>(out_a, out_b, ext0, ext1, tv, bk, rots, rot0, sh, dc, dp, B, st);
+        case 9 * 4 + 2: return launch_cluster_t<9, 2>(out_a, out_b, ext0, ext1, tv, bk, rots, rot0, sh, dc, dp, B, st);
+        case 10 * 4 + 1: return launch_cluster_t<10, 1>(out_a, out_b, ext0, ext1, tv, bk, rots, rot0, sh, dc, dp, B, st);
+        case 10 * 4 + 2: return launch_cluster_t<10, 2>(out_a, out_b, ext0, ext1, tv, bk, rots, rot0, sh, dc, dp, B, st);
+        case 11 * 4 + 1: return launch_cluster_t<11, 1>(out_a, out_b, ext0, ext1, tv, bk, rots, rot0, sh, dc, dp, B, st);
+        case 11 * 4 + 2: return launch_cluster_t<11, 2>(out_a, out_b, ext0, ext1, tv, bk, rots, rot0, sh, dc, dp, B, st);
+        default: return -1;
+    }
+}
+
+// ---- one CMUX step's external product in one launch
+//
+// Block (extended prime e, LWE b): the 2 L0 digits of acc X^r - acc modulo prime e (group d
+// of 2^(K-4) threads reads digit d's limb of the accumulator through L2), their transforms,
+// the products with limb e of the key, and both outputs' inverse transforms into
+// ext [B][2][L0 + 1][N].  Only the accumulator, the key and ext pass through L2; as four
+// launches (rotation difference, transforms, products, inverse) the digits and their spectra
+// did too.  Bound by the FP64 pipe's latency and rate: 1.1 M operations per LWE and step at
+// N = 1024, L0 = 2, 9 us of one SM.  1024 bootstraps at n = 630: 99 ms before, 73 ms.
+template <int K, int L0>
+struct StepShape {
+    static constexpr int N = 1 << K, NE = L0 + 1, ND = 2 * L0, TPT = 1 << (K - 4), THREADS = ND * TPT;
+    static constexpr int PADDED = N + (N >> 4);
+    static constexpr size_t smem = 8 * (size_t)(ND * PADDED);
+    static constexpr int min_ctas = THREADS <= 256 ? 768 / THREADS < 6 ? 768 / THREADS : 6 : 1;  // 85 registers
+};
+
+template <int K, int L0>
+__global__ void __launch_bounds__(StepShape<K, L0>::THREADS, StepShape<K, L0>::min_ctas)
+    k_cggi_step(uint64_t* __restrict__ ext, const uint64_t* __restrict__ acc, const uint64_t* __restrict__ key0,
+                const uint32_t* __restrict__ rots_step, const __grid_constant__ CggiShape sh,
+                const PrimeInfo* __restrict__ primes, int B) {
+    using C = StepShape<K, L0>;
+    constexpr int N = C::N, NE = C::NE, ND = C::ND, TPT = C::TPT, T = C::THREADS, PADDED = C::PADDED;
+    extern __shared__ __align__(128) double sm[];
+    // the blocks of one prime are neighbours: an SM's blocks then share its limb of the key in L1
+    const int e = blockIdx.x / B, b = blockIdx.x - e * B;
+    const int tid = threadIdx.x, g = tid / TPT, t = tid - g * TPT;
+    const PrimeInfo& pi = primes[sh.ext_prime[e]];
+    const double q = pi.qd, qinv = pi.qinv;
+    const FCtx fc = fwd_ctx(pi);
+    double* smg = sm + g * PADDED;
+    const uint64_t* key = key0 + (long long)e * N;
+    double x[16];
+    {
+        PassTw<K - 4, K - 1, K - 4> tw1;
+        f_fwd_tw<K, K - 4, K - 1, K - 4>(tw1, t, 0, K, fc);
+        // digit g: limb g % L0 of component g / L0 of acc X^r - acc (mgsw_CMUX's in2 - in1, mgsw.c:60-61)
+        const int dl = g % L0;
+        const uint64_t ql = primes[sh.lwe_prime[dl]].q;
+        const uint64_t* a = acc + ((long long)b * ND + g) * N;
+        const uint32_t r = rots_step[b];
+#pragma unroll
+        for (int m = 0; m < 16; ++m) {
+            const int j = own<K - 4>(t, m);
+            const uint32_t s = ((uint32_t)j + 2 * N - r) & (2 * N - 1);
+            const uint64_t v = __ldg(a + (s & (N - 1))), u = __ldg(a + j);
+            uint64_t d = s < (uint32_t)N ? v - u : 0 - v - u;
+            // d is in (-2q, q) modulo 2^64
+            if ((long long)d < 0) d += ql;
+            if ((long long)d < 0) d += ql;
+            x[m] = f_from_u64(d);
+            if (dl != e) x[m] = f_reduce(x[m], q, qinv);
+        }
+        tile_fwd_passes<K, true>(fc, K, 0, smg, t, x, tw1, g);
+    }
+    tile_sync<K, true>(g);  // the last exchange is read
+#pragma unroll
+    for (int m = 0; m < 16; ++m) smg[pad(16 * t + m)] = f_reduce(x[m], q, qinv);
+    __syncthreads();
+    // both outputs at two positions a turn: sums of ND products, |sum| <= 3q
+    constexpr int TURNS = N / (2 * T);
+    double s[TURNS][2][2];
+#pragma unroll
+    for (int k = 0; k < TURNS; ++k) {
+        const int xx = 2 * (tid + k * T);
+        s[k][0][0] = s[k][0][1] = s[k][1][0] = s[k][1][1] = 0.0;
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+            const ulonglong2 ka = __ldg(reinterpret_cast<const ulonglong2*>(key + (long long)(2 * d) * NE * N + xx));
+            const ulonglong2 kb = __ldg(reinterpret_cast<const ulonglong2*>(key + (long long)(2 * d + 1) * NE * N + xx));
+            const double v0 = sm[d * PADDED + pad(xx)], v1 = sm[d * PADDED + pad(xx + 1)];
+            const double w0 = __dmul_rn(v0, qinv), w1 = __dmul_rn(v1, qinv);
+            s[k][0][0] = __dadd_rn(s[k][0][0], f_mulmod(f_from_u64(ka.x), v0, w0, q));
+            s[k][0][1] = __dadd_rn(s[k][0][1], f_mulmod(f_from_u64(ka.y), v1, w1, q));
+            s[k][1][0] = __dadd_rn(s[k][1][0], f_mulmod(f_from_u64(kb.x), v0, w0, q));
+            s[k][1][1] = __dadd_rn(s[k][1][1], f_mulmod(f_from_u64(kb.y), v1, w1, q));
+        }
+    }
+    __syncthreads();  // every spectrum is read
+#pragma unroll
+    for (int k = 0; k < TURNS; ++k) {
+        const int xx = 2 * (tid + k * T);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            sm[c * PADDED + pad(xx)] = f_reduce(s[k][c][0], q, qinv);
+            sm[c * PADDED + pad(xx + 1)] = f_reduce(s[k][c][1], q, qinv);
+        }
+    }
+    __syncthreads();
+    if (g >= 2) return;
+#pragma unroll
+    for (int m = 0; m < 16; ++m) x[m] = smg[pad(16 * t + m)];
+    tile_inv_regs<K, true, true>(pi, K, 0, smg, t, x, g);
+    uint64_t* o = ext + (((long long)b * 2 + g) * NE + e) * N;
+#pragma unroll
+    for (int m = 0; m < 16; ++m) o[own<K - 4>(t, m)] = f_to_canonical(x[m], q, qinv, pi.q);
+}
+
+template <int K, int L0>
+int launch_step_t(uint64_t* ext, const uint64_t* acc, const uint64_t* key, const uint32_t* rots_step, const CggiShape& sh,
+                  const PrimeInfo* dp, uint64_t B, cudaStream_t st) {
+    using C = StepShape<K, L0>;
+    if (C::smem > 48 * 1024) {
+        const int e = (int)cudaFuncSetAttribute(k_cggi_step<K, L0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem);
+        if (e) return e;
+    }
+    k_cggi_step<K, L0><<<(unsigned)(B * C::NE), C::THREADS, C::smem, st>>>(ext, acc, key, rots_step, sh, dp, (int)B);
+    note_launch();
+    return (int)cudaGetLastError();
+}
+
+// -1 for shapes without a step kernel.
+int launch_step(int K, uint64_t* ext, const uint64_t* acc, const uint64_t* key, const uint32_t* rots_step,
+                const CggiShape& sh, const PrimeInfo* dp, uint64_t B, cudaStream_t st) {
+    switch (K * 4 + sh.L0) {
+        case 9 * 4 + 1: return launch_step_t<9, 1>(ext, acc, key, rots_step, sh, dp, B, st);
+        case 9 * 4 + 2: return launch_step_t<9, 2>(ext, acc, key, rots_step, sh, dp, B, st);
+        case 10 * 4 + 1: return launch_step_t<10, 1>(ext, acc, key, rots_step, sh, dp, B, st);
+        case 10 * 4 + 2: return launch_step_t<10, 2>(ext, acc, key, rots_step, sh, dp, B, st);
+        case 11 * 4 + 1: return launch_step_t<11, 1>(ext, acc, key, rots_step, sh, dp, B, st);
+        case 11 * 4 + 2: return launch_step_t<11, 2>(ext, acc, key, rots_step, sh, dp, B, st);
+        default: return -1;
+    }
+}
+
 // Sample extraction at coefficient 0 (mlwe.c:40-68): out_a[b][l][i] = a[0] for i = 0,
 // -a[N - i] otherwise; out_b[b][l] = b[0].
 __global__ void k_extract0(uint64_t* __restrict__ out_a, uint64_t* __restrict__ out_b, const uint64_t* __restrict__ acc,
@@ -389,6 +886,15 @@ int cggi_bootstrap(IncNtt* t, uint64_t* out_a, uint64_t* out_b, const uint64_t* 
 
     k_rotations<<<cg_grid(B * (n + 1), 1), 256, 0, st>>>(rots, rot0, in_a, in_b, sh, dp, (long long)B, q0inv,
                                                          (uint64_t)off, (uint64_t)(off >> 64));
+    // The fused kernels take 16-byte key pairs and N = 256 (clusters only) to 2048; one launch
+    // per stage otherwise.  Clusters of one block per SM do best while all of the batch's fit
+    // (44 clusters of 3 do on 148 SMs, 47 do not: 973 and 1519 us at n = 100, where a launch
+    // per step takes 1335); past that the launches, whose blocks never wait for one another.
+    const bool fused = dc.fp64 && t->info[special].fp64 && (reinterpret_cast<uintptr_t>(bk) & 15) == 0;
+    if (fused && B * ne * 9 <= (uint64_t)sm_count() * 8) {
+        const int ec = launch_cluster(t->logP, out_a, out_b, (double*)ext, (double*)D, tv, bk, rots, rot0, sh, dc, dp, B, st);
+        if (ec != -1) return check_cuda(ec, where) ? 0 : 1;
+    }
     k_init_acc<<<cg_grid(N, B * 2 * L0), 256, 0, st>>>(acc, tv, rot0, sh, dp);
     if (!check_cuda(cudaGetLastError(), where)) return 1;
 
@@ -422,6 +928,12 @@ int cggi_bootstrap(IncNtt* t, uint64_t* out_a, uint64_t* out_b, const uint64_t* 
         const uint64_t bk_stride = (uint64_t)nd * 2 * ne * N;
         int err = 0;
         for (uint32_t i = 0; i < n && !err; ++i) {
+            err = fused ? launch_step(t->logP, ext, acc, bk + i * bk_stride, rots + (uint64_t)i * B, sh, dp, B, cs) : -1;
+            if (err == 0) {
+                k_moddown_acc<<<cg_grid((N + 1) / 2, B * 2), 256, 0, cs>>>(acc, ext, sh, dc, dp);
+                continue;
+            }
+            if (err != -1) break;
             // four coefficients per thread: at N = 1024 one block per row, so the launch is
             // not bound by the block rate
             k_rot_diff<<<cg_grid((N + 3) / 4, B * 2 * L0), 256, 0, cs>>>(diff, acc, rots + (uint64_t)i * B, sh, dp);

@@ -334,18 +334,7 @@ __device__ __forceinline__ void tile_sync(int grp) {
     }
 }
 
-// Forward transform of the low K bits of tile r of a 2^logP-point row (16 residues per
-// thread t; the tile's padded exchange buffer at sm); red: reduce each input modulo the
-// row's prime on load.  STAGED: the input was copied into sm by a bulk copy; otherwise
-// it is read from r.src.  tile_fwd_regs leaves the result in x (x[m] at index 16 t + m
-// of the tile, |x| < 2^51, not reduced); tile_fwd_one stores it canonically to r.dst
-// when `store` is set (a thread whose tile only pads out a group computes without
-// storing).  GROUP, grp: the tile's threads synchronise at named barrier 1 + grp
-// (tile_sync).
-template <int K, bool IN_D, bool STAGED, bool GROUP = false>
-__device__ __forceinline__ void tile_fwd_regs(const Tile& r, int logP, bool red, double* sm, int t, double (&x)[16],
-                                              int grp = 0) {
-    const PrimeInfo& pi = *r.pi;
+__device__ __forceinline__ FCtx fwd_ctx(const PrimeInfo& pi) {
     FCtx c;
     c.q = pi.qd;
     c.qinv = pi.qinv;
@@ -353,24 +342,18 @@ __device__ __forceinline__ void tile_fwd_regs(const Tile& r, int logP, bool red,
     c.lt = reinterpret_cast<const double2*>(pi.fwd_lane);
     c.mt = reinterpret_cast<const double2*>(pi.fwd_mid);
     c.lazy = fwd_lazy(pi);
-    const int hi = r.hi;
+    return c;
+}
 
+// The forward passes of one tile whose 16 residues per thread are in x (x[m] at index
+// own<K - 4>(t, m), |x| <= q), the first pass's twiddles in tw1.  On return x[m] is at
+// index 16 t + m (|x| < 2^51, not reduced).
+template <int K, bool GROUP>
+__device__ __forceinline__ void tile_fwd_passes(const FCtx& c, int logP, int hi, double* sm, int t, double (&x)[16],
+                                                const PassTw<K - 4, K - 1, K - 4>& tw1, int grp) {
     constexpr int L1 = K - 4;
     constexpr int L2 = (K - 8) > 0 ? (K - 8) : 0;
     constexpr int L3 = (K - 12) > 0 ? (K - 12) : 0;
-    // each pass's twiddles are requested before the exchange that precedes the pass,
-    // so their latency overlaps the barrier
-    PassTw<L1, K - 1, L1> tw1;
-    f_fwd_tw<K, L1, K - 1, L1>(tw1, t, hi, logP, c);
-    if (STAGED) {
-        const uint64_t* staged = reinterpret_cast<const uint64_t*>(sm);
-#pragma unroll
-        for (int m = 0; m < 16; ++m) x[m] = load_in(staged + own<L1>(t, m), IN_D, red, c);
-        tile_sync<K, GROUP>(grp);  // every input is in registers before the exchanges reuse the buffer
-    } else {
-#pragma unroll
-        for (int m = 0; m < 16; ++m) x[m] = load_in(r.src + own<L1>(t, m), IN_D, red, c);
-    }
     f_fwd_bits<K, L1, K - 1, L1>(x, tw1, c);
     PassTw<L2, L1 - 1, L2> tw2;
     f_fwd_tw<K, L2, L1 - 1, L2>(tw2, t, hi, logP, c);
@@ -396,6 +379,37 @@ __device__ __forceinline__ void tile_fwd_regs(const Tile& r, int logP, bool red,
             f_fwd_bits<K, 0, L3 - 1, 0>(x, tw4, c);
         }
     }
+}
+
+// Forward transform of the low K bits of tile r of a 2^logP-point row (16 residues per
+// thread t; the tile's padded exchange buffer at sm); red: reduce each input modulo the
+// row's prime on load.  STAGED: the input was copied into sm by a bulk copy; otherwise
+// it is read from r.src.  tile_fwd_regs leaves the result in x (x[m] at index 16 t + m
+// of the tile, |x| < 2^51, not reduced); tile_fwd_one stores it canonically to r.dst
+// when `store` is set (a thread whose tile only pads out a group computes without
+// storing).  GROUP, grp: the tile's threads synchronise at named barrier 1 + grp
+// (tile_sync).
+template <int K, bool IN_D, bool STAGED, bool GROUP = false>
+__device__ __forceinline__ void tile_fwd_regs(const Tile& r, int logP, bool red, double* sm, int t, double (&x)[16],
+                                              int grp = 0) {
+    const FCtx c = fwd_ctx(*r.pi);
+    const int hi = r.hi;
+
+    constexpr int L1 = K - 4;
+    // each pass's twiddles are requested before the exchange that precedes the pass,
+    // so their latency overlaps the barrier
+    PassTw<L1, K - 1, L1> tw1;
+    f_fwd_tw<K, L1, K - 1, L1>(tw1, t, hi, logP, c);
+    if (STAGED) {
+        const uint64_t* staged = reinterpret_cast<const uint64_t*>(sm);
+#pragma unroll
+        for (int m = 0; m < 16; ++m) x[m] = load_in(staged + own<L1>(t, m), IN_D, red, c);
+        tile_sync<K, GROUP>(grp);  // every input is in registers before the exchanges reuse the buffer
+    } else {
+#pragma unroll
+        for (int m = 0; m < 16; ++m) x[m] = load_in(r.src + own<L1>(t, m), IN_D, red, c);
+    }
+    tile_fwd_passes<K, GROUP>(c, logP, hi, sm, t, x, tw1, grp);
 }
 
 template <int K, bool IN_D, bool STAGED, bool GROUP = false>
