@@ -673,7 +673,7 @@ __global__ void __launch_bounds__(StepShape<K, L0>::THREADS, StepShape<K, L0>::m
     }
     tile_sync<K, true>(g);  // the last exchange is read
 #pragma unroll
-    for (int m = 0; m < 16; ++m) smg[pad(16 * t + m)] = f_reduce(x[m], q, qinv);
+    for (int m = 0; m < 16; ++m) smg[pad(edge<K>(t, m))] = f_reduce(x[m], q, qinv);
     __syncthreads();
     // both outputs at two positions a turn: sums of ND products, |sum| <= 3q
     constexpr int TURNS = N / (2 * T);
@@ -707,7 +707,7 @@ __global__ void __launch_bounds__(StepShape<K, L0>::THREADS, StepShape<K, L0>::m
     __syncthreads();
     if (g >= 2) return;
 #pragma unroll
-    for (int m = 0; m < 16; ++m) x[m] = smg[pad(16 * t + m)];
+    for (int m = 0; m < 16; ++m) x[m] = smg[pad(edge<K>(t, m))];
     tile_inv_regs<K, true, true>(pi, K, 0, smg, t, x, g);
     uint64_t* o = ext + (((long long)b * 2 + g) * NE + e) * N;
 #pragma unroll

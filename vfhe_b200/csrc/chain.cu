@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(S << (K - 4), (S << (K - 4)) <= 256 ? 2 : 1) k
     constexpr int TPT = 1 << (K - 4), P = 1 << K, PADDED = P + (P >> 4);
     constexpr bool GROUP = S > 1;
     extern __shared__ __align__(128) double csm[];
-    double* spec = csm;            // [S][PADDED]: a's spectra, reduced, at pad(16 t + m)
+    double* spec = csm;            // [S][PADDED]: a's spectra, reduced, at pad(edge<K>(t, m))
     double* ex = csm + S * PADDED;  // [S][PADDED]: each block's exchanges, then b's spectra
     const int g = threadIdx.x / TPT;
     const int t = threadIdx.x - g * TPT;
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(S << (K - 4), (S << (K - 4)) <= 256 ? 2 : 1) k
     tile.src = a + off;
     tile_fwd_regs<K, false, false, GROUP>(tile, K, false, exg, t, x, g);
 #pragma unroll
-    for (int m = 0; m < 16; ++m) spec[g * PADDED + pad(16 * t + m)] = f_reduce(x[m], q, qinv);
+    for (int m = 0; m < 16; ++m) spec[g * PADDED + pad(edge<K>(t, m))] = f_reduce(x[m], q, qinv);
     tile_sync<K, GROUP>(g);  // the block's last exchange reads are over before b's first write
     // b's block g.  Its twiddles are a's again; the prime's address goes through an
     // opaque move so that the compiler reloads them instead of keeping a's ~90 registers
@@ -78,17 +78,17 @@ __global__ void __launch_bounds__(S << (K - 4), (S << (K - 4)) <= 256 ? 2 : 1) k
 #pragma unroll
         for (int m = 0; m < 16; ++m) {
             const double w = f_reduce(x[m], q, qinv);
-            x[m] = f_mulmod(spec[pad(16 * t + m)], w, __dmul_rn(w, qinv), q);  // |x| <= 3q/4
+            x[m] = f_mulmod(spec[pad(edge<K>(t, m))], w, __dmul_rn(w, qinv), q);  // |x| <= 3q/4
         }
     } else {
         tile_sync<K, GROUP>(g);  // the block's exchanges are over: its buffer takes b's spectrum
 #pragma unroll
-        for (int m = 0; m < 16; ++m) exg[pad(16 * t + m)] = f_reduce(x[m], q, qinv);
+        for (int m = 0; m < 16; ++m) exg[pad(edge<K>(t, m))] = f_reduce(x[m], q, qinv);
         __syncthreads();  // every block's spectra of a and b are in shared memory
         const ulonglong2* tw = reinterpret_cast<const ulonglong2*>(pi.twist);
 #pragma unroll
         for (int m = 0; m < 16; ++m) {
-            const int xs = 16 * t + m, px = pad(xs);
+            const int xs = edge<K>(t, m), px = pad(xs);
             double acc = 0.0, wrap = 0.0;
 #pragma unroll
             for (int i = 0; i < S; ++i) {

@@ -184,13 +184,7 @@ __global__ void __launch_bounds__(TileThreads<K>::value) k_fused_fwd_f(const __g
     const int t = threadIdx.x;
     const Tile r = locate<TABLE>(rows, primes, K, row * C + rank, C);
     const PrimeInfo& pi = *r.pi;
-    FCtx c;
-    c.q = pi.qd;
-    c.qinv = pi.qinv;
-    c.tw = reinterpret_cast<const double2*>(pi.fwd_d);
-    c.lt = reinterpret_cast<const double2*>(pi.fwd_lane);
-    c.mt = reinterpret_cast<const double2*>(pi.fwd_mid);
-    c.lazy = fwd_lazy(pi);
+    const FCtx c = fwd_ctx(pi);
     const int logP = rows.logP;
     const bool red = rows.reduce_input != 0;
     // phase 1: this CTA's block, natural order, as residues in doubles
@@ -234,39 +228,13 @@ __global__ void __launch_bounds__(TileThreads<K>::value) k_fused_fwd_f(const __g
     const int hi = rank;
     double x[16];
     constexpr int L1 = K - 4;
-    constexpr int L2 = (K - 8) > 0 ? (K - 8) : 0;
-    constexpr int L3 = (K - 12) > 0 ? (K - 12) : 0;
     PassTw<L1, K - 1, L1> tw1;
     f_fwd_tw<K, L1, K - 1, L1>(tw1, t, hi, logP, c);
 #pragma unroll
     for (int m = 0; m < 16; ++m) x[m] = fsm[own<L1>(t, m)];
     __syncthreads();  // every value is in registers before the exchanges reuse the buffer
-    f_fwd_bits<K, L1, K - 1, L1>(x, tw1, c);
-    PassTw<L2, L1 - 1, L2> tw2;
-    f_fwd_tw<K, L2, L1 - 1, L2>(tw2, t, hi, logP, c);
-    fput<L1>(fsm, x, t);
-    __syncthreads();
-    fget<L2>(x, fsm, t);
-    f_fwd_bits<K, L2, L1 - 1, L2>(x, tw2, c);
-    if constexpr (L2 > 0) {
-        PassTw<L3, L2 - 1, L3> tw3;
-        f_fwd_tw<K, L3, L2 - 1, L3>(tw3, t, hi, logP, c);
-        __syncthreads();
-        fput<L2>(fsm, x, t);
-        __syncthreads();
-        fget<L3>(x, fsm, t);
-        f_fwd_bits<K, L3, L2 - 1, L3>(x, tw3, c);
-        if constexpr (L3 > 0) {
-            PassTw<0, L3 - 1, 0> tw4;
-            f_fwd_tw<K, 0, L3 - 1, 0>(tw4, t, hi, logP, c);
-            __syncthreads();
-            fput<L3>(fsm, x, t);
-            __syncthreads();
-            fget<0>(x, fsm, t);
-            f_fwd_bits<K, 0, L3 - 1, 0>(x, tw4, c);
-        }
-    }
-    store16_canonical(r.dst + 16 * t, x, c.q, c.qinv, pi.q);
+    tile_fwd_passes<K, false>(c, logP, hi, fsm, t, x, tw1, 0);
+    store_edge_canonical<K>(r.dst, x, t, c.q, c.qinv, pi.q);
 }
 
 template <int K, int K1, bool TABLE>
@@ -289,52 +257,8 @@ __global__ void __launch_bounds__(TileThreads<K>::value) k_fused_inv_f(const __g
     const int logP = rows.logP, hi = rank;
     // phase 1: inverse tile passes over the low K bits of this block
     double x[16];
-    constexpr int F1 = 4 < (K - 4) ? 4 : (K - 4);
-    constexpr int F2 = 8 < (K - 4) ? 8 : (K - 4);
-    constexpr int F3 = 12 < (K - 4) ? 12 : (K - 4);
-    load16_u64(x, r.src + 16 * t);
-    PassTw<0, 0, 3> tw1;
-    f_inv_tw<K, 0, 0, 3, false>(tw1, t, hi, logP, c);
-    f_inv_bits<K, 0, 0, 3, false>(x, tw1, c, pi);
-    if constexpr (K <= 8) {
-        PassTw<F1, 4, K - 1> tw2;
-        f_inv_tw<K, F1, 4, K - 1, false>(tw2, t, hi, logP, c);
-        fput<0>(fsm, x, t);
-        __syncthreads();
-        fget<F1>(x, fsm, t);
-        f_inv_bits<K, F1, 4, K - 1, false>(x, tw2, c, pi);
-    } else {
-        PassTw<F1, 4, 7> tw2;
-        f_inv_tw<K, F1, 4, 7, false>(tw2, t, hi, logP, c);
-        fput<0>(fsm, x, t);
-        __syncthreads();
-        fget<F1>(x, fsm, t);
-        f_inv_bits<K, F1, 4, 7, false>(x, tw2, c, pi);
-        if constexpr (K <= 12) {
-            PassTw<F2, 8, K - 1> tw3;
-            f_inv_tw<K, F2, 8, K - 1, false>(tw3, t, hi, logP, c);
-            __syncthreads();
-            fput<F1>(fsm, x, t);
-            __syncthreads();
-            fget<F2>(x, fsm, t);
-            f_inv_bits<K, F2, 8, K - 1, false>(x, tw3, c, pi);
-        } else {
-            PassTw<F2, 8, 11> tw3;
-            f_inv_tw<K, F2, 8, 11, false>(tw3, t, hi, logP, c);
-            __syncthreads();
-            fput<F1>(fsm, x, t);
-            __syncthreads();
-            fget<F2>(x, fsm, t);
-            f_inv_bits<K, F2, 8, 11, false>(x, tw3, c, pi);
-            PassTw<F3, 12, K - 1> tw4;
-            f_inv_tw<K, F3, 12, K - 1, false>(tw4, t, hi, logP, c);
-            __syncthreads();
-            fput<F2>(fsm, x, t);
-            __syncthreads();
-            fget<F3>(x, fsm, t);
-            f_inv_bits<K, F3, 12, K - 1, false>(x, tw4, c, pi);
-        }
-    }
+    load_edge_u64<K>(x, r.src, t);
+    tile_inv_regs<K, false>(pi, logP, hi, fsm, t, x);
     constexpr int LAST = K - 4;
     __syncthreads();  // the exchanges are over: the block goes back in natural order
 #pragma unroll

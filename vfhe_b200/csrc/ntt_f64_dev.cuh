@@ -45,17 +45,35 @@ __device__ __forceinline__ int lane_tw_index(int g, int b, int h) {
     return (((g >> 5) * 15 + ((1 << (3 - b)) - 1) + h) << 5) + (g & 31);
 }
 
-// A thread's 16 consecutive residues (p = row + 16 t): 32-byte accesses when the row is
-// 32-byte aligned (a warp then touches each sector once per instruction), else 16-byte.
-__device__ __forceinline__ void load16_u64(double (&x)[16], const uint64_t* p) {
-    if ((reinterpret_cast<uintptr_t>(p) & 31) == 0) {
+// Stages of a tile's pass at bit 0 (the forward transform's last, the inverse's first): the
+// others take four each.
+template <int K>
+struct EdgePass {
+    static constexpr int NST = (K - 1) % 4 + 1;
+};
+
+// Residue m of thread t in the pass at bit 0: the pass's NST bits and the index's top 4 - NST
+// bits, so that neighbouring lanes own neighbouring groups of 2^NST residues and a warp's
+// global accesses are contiguous (16 consecutive residues a thread when NST = 4: lanes 128
+// bytes apart, 52 L1 wavefronts a 32-byte store against 8).
+template <int K>
+__device__ __forceinline__ int edge(int t, int m) {
+    constexpr int NST = EdgePass<K>::NST;
+    return ((m >> NST) << (K - 4 + NST)) | (t << NST) | (m & ((1 << NST) - 1));
+}
+
+// A thread's 16 residues in the edge layout from / to the tile at p: groups of four as one
+// 32-byte access when the tile is 32-byte aligned, 16-byte accesses otherwise.
+template <int K>
+__device__ __forceinline__ void load_edge_u64(double (&x)[16], const uint64_t* p, int t) {
+    if (EdgePass<K>::NST >= 2 && (reinterpret_cast<uintptr_t>(p) & 31) == 0) {
 #pragma unroll
         for (int m = 0; m < 16; m += 4) {
             uint64_t a, b, c, d;
             // ordered like an ordinary load: rows may be transformed in place
             asm volatile("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];"
                          : "=l"(a), "=l"(b), "=l"(c), "=l"(d)
-                         : "l"(p + m)
+                         : "l"(p + edge<K>(t, m))
                          : "memory");
             x[m] = f_from_u64(a);
             x[m + 1] = f_from_u64(b);
@@ -63,35 +81,34 @@ __device__ __forceinline__ void load16_u64(double (&x)[16], const uint64_t* p) {
             x[m + 3] = f_from_u64(d);
         }
     } else {
-        const ulonglong2* in = reinterpret_cast<const ulonglong2*>(p);
 #pragma unroll
         for (int m = 0; m < 16; m += 2) {
-            const ulonglong2 v = in[m / 2];
+            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p + edge<K>(t, m));
             x[m] = f_from_u64(v.x);
             x[m + 1] = f_from_u64(v.y);
         }
     }
 }
 
-// Canonical residues of x[0..15] to p[0..15] (same access widths as load16_u64).
-__device__ __forceinline__ void store16_canonical(uint64_t* p, const double (&x)[16], double q, double qinv,
-                                                  uint64_t qi) {
-    if ((reinterpret_cast<uintptr_t>(p) & 31) == 0) {
+template <int K>
+__device__ __forceinline__ void store_edge_canonical(uint64_t* p, const double (&x)[16], int t, double q, double qinv,
+                                                     uint64_t qi) {
+    if (EdgePass<K>::NST >= 2 && (reinterpret_cast<uintptr_t>(p) & 31) == 0) {
 #pragma unroll
         for (int m = 0; m < 16; m += 4) {
             const uint64_t a = f_to_canonical(x[m], q, qinv, qi), b = f_to_canonical(x[m + 1], q, qinv, qi);
             const uint64_t c = f_to_canonical(x[m + 2], q, qinv, qi), d = f_to_canonical(x[m + 3], q, qinv, qi);
-            asm volatile("st.global.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(p + m), "l"(a), "l"(b), "l"(c), "l"(d)
+            asm volatile("st.global.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(p + edge<K>(t, m)), "l"(a), "l"(b), "l"(c),
+                         "l"(d)
                          : "memory");
         }
     } else {
-        ulonglong2* out = reinterpret_cast<ulonglong2*>(p);
 #pragma unroll
         for (int m = 0; m < 16; m += 2) {
             ulonglong2 v;
             v.x = f_to_canonical(x[m], q, qinv, qi);
             v.y = f_to_canonical(x[m + 1], q, qinv, qi);
-            out[m / 2] = v;
+            *reinterpret_cast<ulonglong2*>(p + edge<K>(t, m)) = v;
         }
     }
 }
@@ -100,6 +117,7 @@ __device__ __forceinline__ void store16_canonical(uint64_t* p, const double (&x)
 // b = LO + bb uses index (... + (i >> (b+1))), which depends on m only through
 // h = m >> (bb+1): stage bb needs 2^(3-bb) twiddles, a 4-stage pass 15.  Descending
 // (forward) stages are stored first-stage-first; ascending (inverse) the same way.
+// (The pass at bit 0 has fewer stages and its residues' top bits are the index's: EdgePass.)
 template <int LO, int BFROM, int BTO>
 struct PassTw {
     __host__ __device__ static constexpr int count() {
@@ -119,17 +137,41 @@ struct PassTw {
     double2 w[count()];
 };
 
+// Twiddles of the pass at bit 0, stage b, into w[0 .. 2^(3-b)): the lane-major copy (`lt`)
+// for four stages, else the table itself, whose lookups by neighbouring lanes are
+// neighbours in the edge layout; pairs as one 32-byte load.
+template <int K>
+__device__ __forceinline__ void edge_tw(double2* w, int b, int t, int hi, int logP, const FCtx& c) {
+    constexpr int NST = EdgePass<K>::NST;
+    if constexpr (NST == 4) {
+        // one twiddle per thread and slot: the lane-major copy keeps the warp's loads contiguous
+        const int g = (hi << (K - 4)) + t;
+#pragma unroll
+        for (int h = 0; h < (1 << (3 - b)); ++h) w[h] = __ldg(&c.lt[lane_tw_index(g, b, h)]);
+    } else {
+        const double2* T = c.tw + (1 << (logP - 1 - b)) + (hi << (K - b - 1));
+#pragma unroll
+        for (int h = 0; h < (1 << (3 - b)); ++h) {
+            const double2* p = T + (edge<K>(t, h << (b + 1)) >> (b + 1));
+            if (b < NST - 1) {  // slots h and h + 1 are neighbours
+                if (h & 1) continue;
+                asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+                    : "=d"(w[h].x), "=d"(w[h].y), "=d"(w[h + 1].x), "=d"(w[h + 1].y)
+                    : "l"(p));
+            } else {
+                w[h] = __ldg(p);
+            }
+        }
+    }
+}
+
 template <int K, int LO, int BHI, int BLO>
 __device__ __forceinline__ void f_fwd_tw(PassTw<LO, BHI, BLO>& T, int t, int hi, int logP, const FCtx& c) {
 #pragma unroll
     for (int b = BHI; b >= BLO; --b) {
         const int bb = b - LO;
         if constexpr (LO == 0) {
-            // one twiddle per thread and slot: the lane-major copy keeps the warp's loads contiguous
-            const int g = (hi << (K - 4)) + t;
-#pragma unroll
-            for (int h = 0; h < (1 << (3 - bb)); ++h)
-                T.w[PassTw<LO, BHI, BLO>::offset(b) + h] = __ldg(&c.lt[lane_tw_index(g, b, h)]);
+            edge_tw<K>(&T.w[PassTw<LO, BHI, BLO>::offset(b)], b, t, hi, logP, c);
         } else if constexpr (LO == 2 && K >= 6) {
             // four threads per 64-residue group: a warp's loads are 8 consecutive pairs
             const int g = (hi << (K - 6)) + (t >> 2);
@@ -180,10 +222,7 @@ __device__ __forceinline__ void f_inv_tw(PassTw<LO, BLO, BHI>& T, int t, int hi,
         if (FINAL && b == BHI) break;  // the last stage uses the P^-1 constants
         const int bb = b - LO;
         if constexpr (LO == 0) {
-            const int g = (hi << (K - 4)) + t;
-#pragma unroll
-            for (int h = 0; h < (1 << (3 - bb)); ++h)
-                T.w[PassTw<LO, BLO, BHI>::offset(b) + h] = __ldg(&c.lt[lane_tw_index(g, b, h)]);
+            edge_tw<K>(&T.w[PassTw<LO, BLO, BHI>::offset(b)], b, t, hi, logP, c);
         } else if constexpr (LO == 2 && K >= 6) {
             const int g = (hi << (K - 6)) + (t >> 2);
 #pragma unroll
@@ -230,16 +269,17 @@ __device__ __forceinline__ void f_inv_bits(double (&x)[16], const PassTw<LO, BLO
     }
 }
 
-template <int LO>
-__device__ __forceinline__ void fput(double* sm, const double (&x)[16], int t) {
+// Exchange reads and writes in the layout of the pass at LO (the edge layout at bit 0).
+template <int K, int LO>
+__device__ __forceinline__ void fput_at(double* sm, const double (&x)[16], int t) {
 #pragma unroll
-    for (int m = 0; m < 16; ++m) sm[pad(own<LO>(t, m))] = x[m];
+    for (int m = 0; m < 16; ++m) sm[pad(LO == 0 ? edge<K>(t, m) : own<LO>(t, m))] = x[m];
 }
 
-template <int LO>
-__device__ __forceinline__ void fget(double (&x)[16], const double* sm, int t) {
+template <int K, int LO>
+__device__ __forceinline__ void fget_at(double (&x)[16], const double* sm, int t) {
 #pragma unroll
-    for (int m = 0; m < 16; ++m) x[m] = sm[pad(own<LO>(t, m))];
+    for (int m = 0; m < 16; ++m) x[m] = sm[pad(LO == 0 ? edge<K>(t, m) : own<LO>(t, m))];
 }
 
 struct Tile {
@@ -347,7 +387,7 @@ __device__ __forceinline__ FCtx fwd_ctx(const PrimeInfo& pi) {
 
 // The forward passes of one tile whose 16 residues per thread are in x (x[m] at index
 // own<K - 4>(t, m), |x| <= q), the first pass's twiddles in tw1.  On return x[m] is at
-// index 16 t + m (|x| < 2^51, not reduced).
+// index edge<K>(t, m) (|x| < 2^51, not reduced).
 template <int K, bool GROUP>
 __device__ __forceinline__ void tile_fwd_passes(const FCtx& c, int logP, int hi, double* sm, int t, double (&x)[16],
                                                 const PassTw<K - 4, K - 1, K - 4>& tw1, int grp) {
@@ -357,25 +397,25 @@ __device__ __forceinline__ void tile_fwd_passes(const FCtx& c, int logP, int hi,
     f_fwd_bits<K, L1, K - 1, L1>(x, tw1, c);
     PassTw<L2, L1 - 1, L2> tw2;
     f_fwd_tw<K, L2, L1 - 1, L2>(tw2, t, hi, logP, c);
-    fput<L1>(sm, x, t);
+    fput_at<K, L1>(sm, x, t);
     tile_sync<K, GROUP>(grp);
-    fget<L2>(x, sm, t);
+    fget_at<K, L2>(x, sm, t);
     f_fwd_bits<K, L2, L1 - 1, L2>(x, tw2, c);
     if constexpr (L2 > 0) {
         PassTw<L3, L2 - 1, L3> tw3;
         f_fwd_tw<K, L3, L2 - 1, L3>(tw3, t, hi, logP, c);
         tile_sync<K, GROUP>(grp);
-        fput<L2>(sm, x, t);
+        fput_at<K, L2>(sm, x, t);
         tile_sync<K, GROUP>(grp);
-        fget<L3>(x, sm, t);
+        fget_at<K, L3>(x, sm, t);
         f_fwd_bits<K, L3, L2 - 1, L3>(x, tw3, c);
         if constexpr (L3 > 0) {
             PassTw<0, L3 - 1, 0> tw4;
             f_fwd_tw<K, 0, L3 - 1, 0>(tw4, t, hi, logP, c);
             tile_sync<K, GROUP>(grp);
-            fput<L3>(sm, x, t);
+            fput_at<K, L3>(sm, x, t);
             tile_sync<K, GROUP>(grp);
-            fget<0>(x, sm, t);
+            fget_at<K, 0>(x, sm, t);
             f_fwd_bits<K, 0, L3 - 1, 0>(x, tw4, c);
         }
     }
@@ -384,7 +424,7 @@ __device__ __forceinline__ void tile_fwd_passes(const FCtx& c, int logP, int hi,
 // Forward transform of the low K bits of tile r of a 2^logP-point row (16 residues per
 // thread t; the tile's padded exchange buffer at sm); red: reduce each input modulo the
 // row's prime on load.  STAGED: the input was copied into sm by a bulk copy; otherwise
-// it is read from r.src.  tile_fwd_regs leaves the result in x (x[m] at index 16 t + m
+// it is read from r.src.  tile_fwd_regs leaves the result in x (x[m] at index edge<K>(t, m)
 // of the tile, |x| < 2^51, not reduced); tile_fwd_one stores it canonically to r.dst
 // when `store` is set (a thread whose tile only pads out a group computes without
 // storing).  GROUP, grp: the tile's threads synchronise at named barrier 1 + grp
@@ -417,67 +457,42 @@ __device__ __forceinline__ void tile_fwd_one(const Tile& r, const RowSet& rows, 
                                              int grp = 0) {
     double x[16];
     tile_fwd_regs<K, IN_D, STAGED, GROUP>(r, rows.logP, rows.reduce_input != 0, sm, t, x, grp);
-    if (store) store16_canonical(r.dst + 16 * t, x, r.pi->qd, r.pi->qinv, r.pi->q);
+    if (store) store_edge_canonical<K>(r.dst, x, t, r.pi->qd, r.pi->qinv, r.pi->q);
+}
+
+// Passes of the inverse from bit LO up, four stages each, after the pass below left its
+// residues in layout PREV.
+template <int K, int PREV, int LO, bool FINAL, bool GROUP>
+__device__ __forceinline__ void tile_inv_passes(const PrimeInfo& pi, const FCtx& c, int logP, int hi, double* sm, int t,
+                                                double (&x)[16], int grp) {
+    constexpr bool last = LO + 4 == K;
+    PassTw<LO, LO, LO + 3> tw;
+    f_inv_tw<K, LO, LO, LO + 3, FINAL && last>(tw, t, hi, logP, c);
+    if (PREV > 0) tile_sync<K, GROUP>(grp);  // the previous exchange is read
+    fput_at<K, PREV>(sm, x, t);
+    tile_sync<K, GROUP>(grp);
+    fget_at<K, LO>(x, sm, t);
+    f_inv_bits<K, LO, LO, LO + 3, FINAL && last>(x, tw, c, pi);
+    if constexpr (!last) tile_inv_passes<K, LO, LO + 4, FINAL, GROUP>(pi, c, logP, hi, sm, t, x, grp);
 }
 
 // Inverse passes of the low K bits of one tile whose 16 residues per thread t are in x
-// (x[m] at index 16 t + m, |x| < q; the forward passes leave this layout).  FINAL
+// (x[m] at index edge<K>(t, m), |x| < q; the forward passes leave this layout).  FINAL
 // (K == logP): P^-1 folded in.  On return x[m] is at index own<K - 4>(t, m) of the tile.
 template <int K, bool FINAL, bool GROUP = false>
 __device__ __forceinline__ void tile_inv_regs(const PrimeInfo& pi, int logP, int hi, double* sm, int t,
                                               double (&x)[16], int grp = 0) {
+    constexpr int NST = EdgePass<K>::NST;
     FCtx c;
     c.q = pi.qd;
     c.qinv = pi.qinv;
     c.tw = reinterpret_cast<const double2*>(pi.inv_d);
     c.lt = reinterpret_cast<const double2*>(pi.inv_lane);
     c.mt = reinterpret_cast<const double2*>(pi.inv_mid);
-
-    constexpr int F1 = 4 < (K - 4) ? 4 : (K - 4);
-    constexpr int F2 = 8 < (K - 4) ? 8 : (K - 4);
-    constexpr int F3 = 12 < (K - 4) ? 12 : (K - 4);
-    PassTw<0, 0, 3> tw1;
-    f_inv_tw<K, 0, 0, 3, false>(tw1, t, hi, logP, c);
-    f_inv_bits<K, 0, 0, 3, false>(x, tw1, c, pi);
-    if constexpr (K <= 8) {
-        PassTw<F1, 4, K - 1> tw2;
-        f_inv_tw<K, F1, 4, K - 1, FINAL>(tw2, t, hi, logP, c);
-        fput<0>(sm, x, t);
-        tile_sync<K, GROUP>(grp);
-        fget<F1>(x, sm, t);
-        f_inv_bits<K, F1, 4, K - 1, FINAL>(x, tw2, c, pi);
-    } else {
-        PassTw<F1, 4, 7> tw2;
-        f_inv_tw<K, F1, 4, 7, false>(tw2, t, hi, logP, c);
-        fput<0>(sm, x, t);
-        tile_sync<K, GROUP>(grp);
-        fget<F1>(x, sm, t);
-        f_inv_bits<K, F1, 4, 7, false>(x, tw2, c, pi);
-        if constexpr (K <= 12) {
-            PassTw<F2, 8, K - 1> tw3;
-            f_inv_tw<K, F2, 8, K - 1, FINAL>(tw3, t, hi, logP, c);
-            tile_sync<K, GROUP>(grp);
-            fput<F1>(sm, x, t);
-            tile_sync<K, GROUP>(grp);
-            fget<F2>(x, sm, t);
-            f_inv_bits<K, F2, 8, K - 1, FINAL>(x, tw3, c, pi);
-        } else {
-            PassTw<F2, 8, 11> tw3;
-            f_inv_tw<K, F2, 8, 11, false>(tw3, t, hi, logP, c);
-            tile_sync<K, GROUP>(grp);
-            fput<F1>(sm, x, t);
-            tile_sync<K, GROUP>(grp);
-            fget<F2>(x, sm, t);
-            f_inv_bits<K, F2, 8, 11, false>(x, tw3, c, pi);
-            PassTw<F3, 12, K - 1> tw4;
-            f_inv_tw<K, F3, 12, K - 1, FINAL>(tw4, t, hi, logP, c);
-            tile_sync<K, GROUP>(grp);
-            fput<F2>(sm, x, t);
-            tile_sync<K, GROUP>(grp);
-            fget<F3>(x, sm, t);
-            f_inv_bits<K, F3, 12, K - 1, FINAL>(x, tw4, c, pi);
-        }
-    }
+    PassTw<0, 0, NST - 1> tw1;
+    f_inv_tw<K, 0, 0, NST - 1, false>(tw1, t, hi, logP, c);
+    f_inv_bits<K, 0, 0, NST - 1, false>(x, tw1, c, pi);
+    tile_inv_passes<K, 0, NST, FINAL, GROUP>(pi, c, logP, hi, sm, t, x, grp);
 }
 
 // Inverse transform of the low K bits of tile r.  FINAL (K == logP): P^-1 folded in,
@@ -489,15 +504,15 @@ __device__ __forceinline__ void tile_inv_one(const Tile& r, const RowSet& rows, 
     const PrimeInfo& pi = *r.pi;
     double x[16];
     if (STAGED) {
-        const ulonglong2* in = reinterpret_cast<const ulonglong2*>(reinterpret_cast<const uint64_t*>(sm) + 16 * t);
+        const uint64_t* in = reinterpret_cast<const uint64_t*>(sm);
 #pragma unroll
         for (int m = 0; m < 16; m += 2) {
-            const ulonglong2 v = in[m / 2];
+            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(in + edge<K>(t, m));
             x[m] = f_from_u64(v.x);
             x[m + 1] = f_from_u64(v.y);
         }
     } else {
-        load16_u64(x, r.src + 16 * t);
+        load_edge_u64<K>(x, r.src, t);
     }
     if (STAGED) tile_sync<K, GROUP>(grp);  // every input is in registers before the exchanges reuse the buffer
     tile_inv_regs<K, FINAL, GROUP>(pi, rows.logP, r.hi, sm, t, x, grp);
