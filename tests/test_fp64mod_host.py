@@ -108,3 +108,21 @@ def test_centred_twiddle_with_lazy_input(q):
             t = f_mulmod(float(y), fw, wq, qd)
             assert t == int(t) and abs(t) <= 0.75 * q, (y, w)
             assert (int(t) - y * w) % q == 0, (y, w)
+
+
+@pytest.mark.parametrize("q", [(1 << 50) - 27, (1 << 49) + 1, (1 << 47) + 5])
+def test_six_butterfly_stages_without_a_reduction(q):
+    """Forward stages from |x| <= q/2 + 1: a stage adds at most q/2 + q |x| 2^-54 to |x|,
+    so the product's operand stays below 2^52 for six stages, and the canonical
+    store reduces what they leave (below 4.3 q)."""
+    rng = np.random.default_rng(13)
+    qd = float(q)
+    qinv = 1.0 / qd
+    top = q // 2 + 1
+    for _ in range(6):
+        assert top < 1 << 52
+        top += q // 2 + (q * top >> 54) + 2
+    assert top < 4.3 * q and top < 1 << 53
+    for x in [top, -top, top - 1, 4 * q, -4 * q, 4 * q + q // 2, 3 * q + q // 2 + 1] + \
+            [int(v) for v in rng.integers(-top, top, 200)]:
+        assert f_to_canonical(float(x), qd, qinv, q) == x % q, x

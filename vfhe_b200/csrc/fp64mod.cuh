@@ -31,7 +31,8 @@ __device__ __forceinline__ double f_mulmod(double y, double w, double wq, double
     return __dadd_rn(r, l);
 }
 
-// x mod q, centred, |result| <= q/2 + 1 (needs |x| < 2^52 and qinv = fl(1/q)).
+// x mod q, centred, |result| <= q/2 + 1 (needs |x| < 2^53 an exact integer, |x| < 8 q or |x| <
+// 2^52, and qinv = fl(1/q): x - n q is then exact).
 __device__ __forceinline__ double f_reduce(double x, double q, double qinv) {
     const double n = __dadd_rn(__fma_rn(x, qinv, kRoundMagic), -kRoundMagic);
     return __fma_rn(-n, q, x);

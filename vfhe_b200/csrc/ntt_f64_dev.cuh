@@ -5,7 +5,8 @@
 //
 // Range schedule (every modular product needs its input below 2^52 in magnitude):
 //   forward (CT: x +- w y): each stage adds at most 3q/4, so passes of <= 4 stages
-//     starting from |x| <= q stay below 4q; all residues are reduced at pass end;
+//     starting from |x| <= q stay below 4q; all residues are reduced at pass end unless
+//     at most two stages follow (f_fwd_bits);
 //   inverse (GS: x + y, w (x - y)): sums double, so the sum outputs are reduced after
 //     every second stage and at pass end; products are always <= 3q/4.
 #pragma once
@@ -19,11 +20,22 @@ namespace vc {
 
 namespace {
 
-__device__ __forceinline__ int pad(int i) { return i + (i >> 4); }
+__host__ __device__ __forceinline__ constexpr int pad(int i) { return i + (i >> 4); }
 
+// Residue m of thread t in the pass over bits LO..LO+3: place own_base + own_step.  The two
+// have no bits in common, so pads and shifts of the place split into the thread's part and a
+// constant per m (an immediate offset): pad(i | j) = pad(i) + pad(j).
+template <int LO>
+__device__ __forceinline__ int own_base(int t) {
+    return ((t >> LO) << (LO + 4)) | (t & ((1 << LO) - 1));
+}
+template <int LO>
+__host__ __device__ __forceinline__ constexpr int own_step(int m) {
+    return m << LO;
+}
 template <int LO>
 __device__ __forceinline__ int own(int t, int m) {
-    return ((t >> LO) << (LO + 4)) | (m << LO) | (t & ((1 << LO) - 1));
+    return own_base<LO>(t) + own_step<LO>(m);
 }
 
 struct FCtx {
@@ -57,9 +69,17 @@ struct EdgePass {
 // global accesses are contiguous (16 consecutive residues a thread when NST = 4: lanes 128
 // bytes apart, 52 L1 wavefronts a 32-byte store against 8).
 template <int K>
-__device__ __forceinline__ int edge(int t, int m) {
+__device__ __forceinline__ int edge_base(int t) {
+    return t << EdgePass<K>::NST;
+}
+template <int K>
+__host__ __device__ __forceinline__ constexpr int edge_step(int m) {
     constexpr int NST = EdgePass<K>::NST;
-    return ((m >> NST) << (K - 4 + NST)) | (t << NST) | (m & ((1 << NST) - 1));
+    return ((m >> NST) << (K - 4 + NST)) | (m & ((1 << NST) - 1));
+}
+template <int K>
+__device__ __forceinline__ int edge(int t, int m) {
+    return edge_base<K>(t) + edge_step<K>(m);
 }
 
 // A thread's 16 residues in the edge layout from / to the tile at p: groups of four as one
@@ -152,7 +172,7 @@ __device__ __forceinline__ void edge_tw(double2* w, int b, int t, int hi, int lo
         const double2* T = c.tw + (1 << (logP - 1 - b)) + (hi << (K - b - 1));
 #pragma unroll
         for (int h = 0; h < (1 << (3 - b)); ++h) {
-            const double2* p = T + (edge<K>(t, h << (b + 1)) >> (b + 1));
+            const double2* p = T + (edge_base<K>(t) >> (b + 1)) + (edge_step<K>(h << (b + 1)) >> (b + 1));
             if (b < NST - 1) {  // slots h and h + 1 are neighbours
                 if (h & 1) continue;
                 asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
@@ -179,11 +199,10 @@ __device__ __forceinline__ void f_fwd_tw(PassTw<LO, BHI, BLO>& T, int t, int hi,
             for (int h = 0; h < (1 << (3 - bb)); ++h)
                 T.w[PassTw<LO, BHI, BLO>::offset(b) + h] = __ldg(&c.mt[lane_tw_index(g, bb, h)]);
         } else {
-            const int base = (1 << (logP - 1 - b)) + (hi << (K - b - 1));
+            const double2* p = c.tw + (1 << (logP - 1 - b)) + (hi << (K - b - 1)) + (own_base<LO>(t) >> (b + 1));
 #pragma unroll
             for (int h = 0; h < (1 << (3 - bb)); ++h)
-                T.w[PassTw<LO, BHI, BLO>::offset(b) + h] =
-                    __ldg(&c.tw[base + (own<LO>(t, h << (bb + 1)) >> (b + 1))]);
+                T.w[PassTw<LO, BHI, BLO>::offset(b) + h] = __ldg(p + (own_step<LO>(h << (bb + 1)) >> (b + 1)));
         }
     }
 }
@@ -203,9 +222,11 @@ __device__ __forceinline__ void f_fwd_bits(double (&x)[16], const PassTw<LO, BHI
             x[m | (1 << bb)] = __dsub_rn(u, v);
         }
     }
-    // The pass at bit 0 is the transform's last and is followed by f_to_canonical, whose
-    // own reduction takes its outputs (|x| < 4q < 2^52) directly.
-    if constexpr (LO != 0) {
+    // A stage takes |x| <= a q to (a + 1/2 + a / 16) q (|t| <= q/2 + q |y| 2^-54, q < 2^50), so
+    // six stages from q/2 keep every product's operand below 3.6 q < 2^52 and end below 4.3 q,
+    // which f_to_canonical's own reduction takes: no reduction before a pass of one or two
+    // stages, the transform's last, and none after it.
+    if constexpr (LO > 2) {
         if (!c.lazy) {
 #pragma unroll
             for (int m = 0; m < 16; ++m) x[m] = f_reduce(x[m], c.q, c.qinv);
@@ -229,11 +250,10 @@ __device__ __forceinline__ void f_inv_tw(PassTw<LO, BLO, BHI>& T, int t, int hi,
             for (int h = 0; h < (1 << (3 - bb)); ++h)
                 T.w[PassTw<LO, BLO, BHI>::offset(b) + h] = __ldg(&c.mt[lane_tw_index(g, bb, h)]);
         } else {
-            const int base = ((1 << logP) >> (b + 1)) + (hi << (K - b - 1));
+            const double2* p = c.tw + ((1 << logP) >> (b + 1)) + (hi << (K - b - 1)) + (own_base<LO>(t) >> (b + 1));
 #pragma unroll
             for (int h = 0; h < (1 << (3 - bb)); ++h)
-                T.w[PassTw<LO, BLO, BHI>::offset(b) + h] =
-                    __ldg(&c.tw[base + (own<LO>(t, h << (bb + 1)) >> (b + 1))]);
+                T.w[PassTw<LO, BLO, BHI>::offset(b) + h] = __ldg(p + (own_step<LO>(h << (bb + 1)) >> (b + 1)));
         }
     }
 }
@@ -271,15 +291,26 @@ __device__ __forceinline__ void f_inv_bits(double (&x)[16], const PassTw<LO, BLO
 
 // Exchange reads and writes in the layout of the pass at LO (the edge layout at bit 0).
 template <int K, int LO>
+__device__ __forceinline__ int slot_base(int t) {
+    return pad(LO == 0 ? edge_base<K>(t) : own_base<LO>(t));
+}
+template <int K, int LO>
+__host__ __device__ __forceinline__ constexpr int slot_step(int m) {
+    return pad(LO == 0 ? edge_step<K>(m) : own_step<LO>(m));
+}
+
+template <int K, int LO>
 __device__ __forceinline__ void fput_at(double* sm, const double (&x)[16], int t) {
+    double* p = sm + slot_base<K, LO>(t);
 #pragma unroll
-    for (int m = 0; m < 16; ++m) sm[pad(LO == 0 ? edge<K>(t, m) : own<LO>(t, m))] = x[m];
+    for (int m = 0; m < 16; ++m) p[slot_step<K, LO>(m)] = x[m];
 }
 
 template <int K, int LO>
 __device__ __forceinline__ void fget_at(double (&x)[16], const double* sm, int t) {
+    const double* p = sm + slot_base<K, LO>(t);
 #pragma unroll
-    for (int m = 0; m < 16; ++m) x[m] = sm[pad(LO == 0 ? edge<K>(t, m) : own<LO>(t, m))];
+    for (int m = 0; m < 16; ++m) x[m] = p[slot_step<K, LO>(m)];
 }
 
 struct Tile {
