@@ -24,14 +24,14 @@ from .native import Engine, cuda_engine
 
 DEFAULT_TABLE = Path(__file__).resolve().parent / "tuned" / "ntt_schedule_b200.json"
 MAX_ELEMS = 1 << 28  # at most 2 GiB of rows per timed buffer
-BUCKETS = (4, 7, 9, 11, 13, 15)
+BUCKETS = tuple(range(4, 16))
 KEEP_DEFAULT_MARGIN = 0.03  # a tuned schedule must beat the built-in one by 3%
 
 
 def candidates(logP: int) -> list[tuple[int, int, int]]:
     """(tile_bits, tiles_per_cta, ctas_per_sm) triples worth timing for one logP."""
     if logP <= 13:  # one pass, or a short column pass in front of smaller tiles
-        tiles = {k for k in (logP, logP - 1, logP - 2) if k >= 8}
+        tiles = {k for k in (logP, logP - 1, logP - 2, logP - 3) if k >= 8}
     else:  # a column pass of radix 2^(logP - k) is required
         tiles = set(range(max(8, logP - 5), 14))
     out = []
