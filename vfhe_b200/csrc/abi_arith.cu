@@ -475,41 +475,64 @@ void polynomial_RNSc_mod_reduce_lifted(void* out, void* in, uint64_t idx) {
 // Sequential division by every prime of `divide_mask` in increasing limb order
 // (rns_polynomial.c:905-976): each step updates every other active limb, including
 // limbs dropped later, then clears the dropped row and its mask bit.
-static void divide(Poly* o, uint64_t divide_mask, bool round, const char* where) {
+// Polynomials of one pool with the same active limbs go together.
+static void divide(Poly* const* polys, int count, uint64_t divide_mask, bool round, const char* where) {
+    Poly* o = polys[0];
     IncNtt* t = pool_of(o);
     uint64_t mask = divide_mask & o->pub.rns_mask;
+    bool together = count <= kDividePolys && count * popcount64(o->pub.rns_mask) <= kMaxLimbs;
+    for (int k = 1; k < count; ++k) {
+        together = together && pool_of(polys[k]) == t && polys[k]->pub.rns_mask == o->pub.rns_mask &&
+                   polys[k]->pub.allocated_l == o->pub.allocated_l;
+        for (int j = 0; j < k; ++j) together = together && polys[j] != polys[k];
+    }
+    if (!together) {
+        for (int k = 0; k < count; ++k) divide(polys + k, 1, divide_mask, round, where);
+        return;
+    }
     if (!mask) return;
-    prefetch_poly(o);
+    for (int k = 0; k < count; ++k) prefetch_poly(polys[k]);
     for (uint64_t idx = 0; idx < o->pub.allocated_l; ++idx) {
         if (!(mask & (1ULL << idx))) continue;
         const uint64_t p = t->info[idx].q;
         DivideArgs d;
-        d.drop_row = o->pub.coeffs[idx];
+        memset(&d, 0, sizeof d);
+        d.polys = count;
         d.half_drop = round ? p / 2 : 0;
         d.p = p;
         d.drop_prime = (uint32_t)idx;
-        EwSet s = poly_set(o, nullptr, nullptr, o->pub.rns_mask & ~(1ULL << idx));
-        for (int k = 0; k < s.nlimbs; ++k) {
-            const uint64_t q = t->info[s.prime[k]].q;
-            s.s[k] = host_inv_mod(p % q, q);
-            s.s_sh[k] = host_shoup(s.s[k], q);
+        EwSet s = empty_set((long long)t->pub.N);
+        for (int k = 0; k < count; ++k) {
+            d.drop_row[k] = polys[k]->pub.coeffs[idx];
+            const EwSet one = poly_set(polys[k], nullptr, nullptr, o->pub.rns_mask & ~(1ULL << idx));
+            for (int j = 0; j < one.nlimbs; ++j) {
+                const int at = s.nlimbs + j;
+                const uint64_t q = t->info[one.prime[j]].q;
+                s.out[at] = one.out[j];
+                s.prime[at] = one.prime[j];
+                s.s[at] = k ? s.s[j] : host_inv_mod(p % q, q);
+                s.s_sh[at] = k ? s.s_sh[j] : host_shoup(s.s[at], q);
+            }
+            s.nlimbs += one.nlimbs;
         }
         if (!check_cuda(launch_divide(s, d, t->d_info, stream()), where)) return;
-        o->pub.rns_mask &= ~(1ULL << idx);
+        for (int k = 0; k < count; ++k) polys[k]->pub.rns_mask &= ~(1ULL << idx);
     }
 }
 
 void polynomial_round_division_RNSc_wo_free(void* out, uint64_t divide_mask) {
     VC_ENTER("polynomial_round_division_RNSc_wo_free");
     if (!valid_poly(out, vc_where_)) return;
-    divide(as_poly(out), divide_mask, true, vc_where_);
+    Poly* o = as_poly(out);
+    divide(&o, 1, divide_mask, true, vc_where_);
     VC_FINISH();
 }
 
 void polynomial_floor_division_RNSc_wo_free(void* out, uint64_t divide_mask) {
     VC_ENTER("polynomial_floor_division_RNSc_wo_free");
     if (!valid_poly(out, vc_where_)) return;
-    divide(as_poly(out), divide_mask, false, vc_where_);
+    Poly* o = as_poly(out);
+    divide(&o, 1, divide_mask, false, vc_where_);
     VC_FINISH();
 }
 
@@ -684,6 +707,12 @@ void op_product(Poly* out, Poly* a, Poly* b, int mode, const char* where) {
 void op_zero_rows(Poly* p, uint64_t rows, const char* where) {
     const uint64_t all = (p->pub.allocated_l >= 64) ? ~0ULL : ((1ULL << p->pub.allocated_l) - 1);
     ew_mask(EW_ZERO, p, nullptr, nullptr, rows & all, where);
+}
+
+void op_round_divide(Poly* const* polys, int count, uint64_t divide_mask, const char* where) {
+    for (int k = 0; k < count; ++k)
+        if (!valid_poly(polys[k], where)) return;
+    if (count > 0) divide(polys, count, divide_mask, true, where);
 }
 
 void op_scale_addto(Poly* out, Poly* a, uint64_t s, const char* where) {

@@ -86,6 +86,9 @@ inline uint64_t host_reduce_signed(uint64_t v, uint64_t q) {
 void op_product(Poly* out, Poly* a, Poly* b, int mode, const char* where);
 // Zero the rows selected by `rows` (limb bit mask) regardless of the active mask.
 void op_zero_rows(Poly* p, uint64_t rows, const char* where);
+// Round division of several polynomials by every prime of divide_mask, in one launch per
+// prime where they share a pool and active limbs.
+void op_round_divide(Poly* const* polys, int count, uint64_t divide_mask, const char* where);
 // out += a * s (per-limb scalar s[limb index]); out's mask becomes a's mask.
 void op_scale_addto(Poly* out, Poly* a, uint64_t s, const char* where);
 

@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "abi_common.cuh"
+#include "fp64mod.cuh"
 
 using namespace vc;
 
@@ -44,20 +45,75 @@ void prefetch_mlwe(RNS_MLWE m) {
     prefetch_poly(P_(m->b));
 }
 
+void set_masks(RNS_MLWE m, uint64_t mask);
+
 uint64_t all_rows(Poly* p) {
     return p->pub.allocated_l >= 64 ? ~0ULL : ((1ULL << p->pub.allocated_l) - 1);
 }
 
-// mlwe_RNS_trivial_sample_of_zero (mlwe.c:302-312): every row of every component zeroed.
-void zero_mlwe(RNS_MLWE m, const char* where) {
-    for (uint64_t i = 0; i < m->r; ++i) op_zero_rows(P_(m->a[i]), all_rows(P_(m->a[i])), where);
-    op_zero_rows(P_(m->b), all_rows(P_(m->b)), where);
+// mlwe_RNS_trivial_sample_of_zero (mlwe.c:302-312): every row of every component zeroed
+// (or the rows of `rows` only).  Components with few rows share a launch.
+void zero_mlwe(RNS_MLWE m, const char* where, uint64_t rows = ~0ULL) {
+    EwSet s = empty_set((long long)m->b->ntt->N);
+    for (uint64_t c = 0; c <= m->r; ++c) {
+        Poly* p = P_(c < m->r ? m->a[c] : m->b);
+        const uint64_t mask = rows & all_rows(p);
+        if (s.nlimbs + popcount64(mask) > kMaxLimbs) {
+            check_cuda(launch_ew(EW_ZERO, s, pool(m)->d_info, stream()), where);
+            s.nlimbs = 0;
+        }
+        const EwSet one = poly_set(p, nullptr, nullptr, mask);
+        for (int k = 0; k < one.nlimbs; ++k) {
+            s.out[s.nlimbs] = one.out[k];
+            s.prime[s.nlimbs++] = one.prime[k];
+        }
+    }
+    if (s.nlimbs) check_cuda(launch_ew(EW_ZERO, s, pool(m)->d_info, stream()), where);
 }
+
+// The transform of every component in one launch, where all components of both samples have
+// one pool and one set of active limbs and their rows fit a row set.  False: nothing done.
+bool transform_together(RNS_MLWE o, RNS_MLWE i, bool inverse, const char* where) {
+    if (!o || !i || o->r != i->r || !o->b || !i->b) return false;
+    IncNtt* t = pool(o);
+    const uint64_t mask = i->b->rns_mask;
+    uint32_t idx[64];
+    const int n = mask_indices(mask, t->pub.l, idx);
+    if (n == 0 || (int)(o->r + 1) * n > kMaxLimbs) return false;
+    RowSet rs;
+    memset(&rs, 0, sizeof rs);
+    for (uint64_t c = 0; c <= o->r; ++c) {
+        Poly* po = P_(c < o->r ? o->a[c] : o->b);
+        Poly* pi = P_(c < i->r ? i->a[c] : i->b);
+        if (!po || !pi || !po->base || !pi->base || pool_of(po) != t || pool_of(pi) != t || pi->pub.rns_mask != mask)
+            return false;
+        if (idx[n - 1] >= po->pub.allocated_l || idx[n - 1] >= pi->pub.allocated_l) return false;
+        for (int k = 0; k < n; ++k) {
+            rs.in[rs.nlimbs] = pi->pub.coeffs[idx[k]];
+            rs.out[rs.nlimbs] = po->pub.coeffs[idx[k]];
+            rs.prime[rs.nlimbs++] = idx[k];
+        }
+    }
+    rs.split = (int)t->pub.split_degree;
+    rs.logP = t->logP;
+    rs.batch = 1;
+    mark_fp64(rs, t);
+    if (!check_cuda(launch_ntt(rs, t->d_info, inverse, stream()), where)) return true;
+    set_masks(o, mask);
+    return true;
+}
+
+bool gadget_all_ok(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly);
+void gadget_mac_all(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly, int mode, const char* where);
 
 // gadget_mul_{add,sub}to_polynomial (gadget.c:5-36): digit j = limb j of the
 // coefficient-domain `poly`, lifted to the key's extended limbs, transformed, and
 // multiplied into `out` with ksk[digit].
 void gadget_mac(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly, int mode, const char* where) {
+    if (gadget_all_ok(out, ksk, poly)) {
+        gadget_mac_all(out, ksk, poly, mode, where);
+        return;
+    }
     IncNtt* t = pool(out);
     Poly* tmp = poly_create(0, ksk[0]->b->rns_mask, reinterpret_cast<IncNtt*>(ksk[0]->b->ntt));
     uint64_t k = 0;
@@ -76,6 +132,229 @@ void set_masks(RNS_MLWE m, uint64_t mask) {
     for (uint64_t i = 0; i < m->r; ++i) m->a[i]->rns_mask = mask;
     m->b->rns_mask = mask;
 }
+
+// ---- gadget products with every digit at once
+//
+// The digits of a polynomial are transformed in one launch (digit mode of a row set) into
+// device scratch and multiplied with the key rows, which stay where their polynomials keep
+// them, in one more.  One digit after the other, each four launches over a few rows, left
+// the GPU idle: a rotation at N = 2^14, 8 limbs, 240 -> 87 us a call; a multiplication with
+// its relinearisation at 9 limbs, 513 -> 319 us (118 with its operands' pages on the device).
+
+constexpr int kGadgetComps = 4;                  // components of a sample (rank + 1) the kernel takes
+constexpr int kGadgetKeys = 192;                 // key polynomials (digits x components) of one launch
+constexpr size_t kGadgetScratch = 64ULL << 20;   // bytes of digit spectra at once
+
+struct GadgetMac {
+    const uint64_t* key[kGadgetKeys];  // block of digit j's component c at j * comps + c; row i at i N
+    uint64_t* out[kGadgetComps];       // block of output component c
+    uint32_t prime[kMaxLimbs];         // pool index of extended limb i
+    int digits, ne;
+    int mode;  // 0: out = sum, 1: out += sum, 2: out -= sum, 3: out = -sum
+};
+
+__device__ __forceinline__ uint64_t gadget_result(double s, uint64_t cur, int mode, const PrimeInfo& pi) {
+    // |s| <= 3.5 q, and a residue
+    if (mode & 2) s = -s;
+    if (mode == 1 || mode == 2) s = __dadd_rn(s, f_from_u64(cur));
+    return f_to_canonical(s, pi.qd, pi.qinv, pi.q);
+}
+
+// D [digits][ne][N].  Exact FP64 as in k_mac: canonical operands below 2^50, |term| <= 3q/4,
+// sums reduced after every fourth.  Split 1: two residues a thread.
+template <int NC>
+__global__ void __launch_bounds__(256) k_gadget_mac1(const __grid_constant__ GadgetMac gm, const uint64_t* __restrict__ D,
+                                                     const PrimeInfo* __restrict__ primes, long long N) {
+    const int i = blockIdx.y;
+    const PrimeInfo& pi = primes[gm.prime[i]];
+    const double q = pi.qd, qinv = pi.qinv;
+    const long long row = (long long)gm.prime[i] * N;
+    for (long long x = 2 * (blockIdx.x * (long long)blockDim.x + threadIdx.x); x < N;
+         x += 2 * (long long)gridDim.x * blockDim.x) {
+        double s0[NC], s1[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) s0[c] = s1[c] = 0.0;
+        for (int j = 0; j < gm.digits; ++j) {
+            const ulonglong2 d = *reinterpret_cast<const ulonglong2*>(D + ((long long)j * gm.ne + i) * N + x);
+            const double v0 = f_from_u64(d.x), v1 = f_from_u64(d.y);
+            const double w0 = __dmul_rn(v0, qinv), w1 = __dmul_rn(v1, qinv);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(gm.key[j * NC + c] + row + x);
+                s0[c] = __dadd_rn(s0[c], f_mulmod(f_from_u64(k.x), v0, w0, q));
+                s1[c] = __dadd_rn(s1[c], f_mulmod(f_from_u64(k.y), v1, w1, q));
+                if ((j & 3) == 3) {
+                    s0[c] = f_reduce(s0[c], q, qinv);
+                    s1[c] = f_reduce(s1[c], q, qinv);
+                }
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            ulonglong2* o = reinterpret_cast<ulonglong2*>(gm.out[c] + row + x);
+            const ulonglong2 cur = *o;
+            ulonglong2 r;
+            r.x = gadget_result(s0[c], cur.x, gm.mode, pi);
+            r.y = gadget_result(s1[c], cur.y, gm.mode, pi);
+            *o = r;
+        }
+    }
+}
+
+// Split S > 1: the incomplete product's block o at slot x (rns_polynomial.c:358-435).
+template <int NC>
+__global__ void __launch_bounds__(256) k_gadget_mac(const __grid_constant__ GadgetMac gm, const uint64_t* __restrict__ D,
+                                                    const PrimeInfo* __restrict__ primes, long long N, int S) {
+    const int i = blockIdx.y;
+    const PrimeInfo& pi = primes[gm.prime[i]];
+    const double q = pi.qd, qinv = pi.qinv;
+    const long long row = (long long)gm.prime[i] * N, P = N / S;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < N; e += (long long)gridDim.x * blockDim.x) {
+        const int o = (int)(e / P);
+        const long long x = e - o * P;
+        double s[NC], w[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) s[c] = w[c] = 0.0;
+        int terms = 0;
+        for (int j = 0; j < gm.digits; ++j)
+            for (int b = 0; b < S; ++b) {
+                const double v = f_from_u64(D[((long long)j * gm.ne + i) * N + b * P + x]);
+                const double vq = __dmul_rn(v, qinv);
+                const bool wrap = b > o;
+                const long long at = row + (wrap ? o - b + S : o - b) * P + x;
+                const bool full = ++terms % 4 == 0;
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const double t = f_mulmod(f_from_u64(gm.key[j * NC + c][at]), v, vq, q);
+                    if (wrap) w[c] = __dadd_rn(w[c], t);
+                    else s[c] = __dadd_rn(s[c], t);
+                    if (full) {
+                        s[c] = f_reduce(s[c], q, qinv);
+                        w[c] = f_reduce(w[c], q, qinv);
+                    }
+                }
+            }
+        const double tw = f_from_u64(reinterpret_cast<const ulonglong2*>(pi.twist)[x].x);
+        const double twq = __dmul_rn(tw, qinv);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const double r = __dadd_rn(f_reduce(s[c], q, qinv), f_mulmod(f_reduce(w[c], q, qinv), tw, twq, q));
+            uint64_t* out = gm.out[c] + row + e;
+            *out = gadget_result(r, *out, gm.mode, pi);
+        }
+    }
+}
+
+template <int NC>
+int launch_gadget_mac(const GadgetMac& gm, const uint64_t* D, const PrimeInfo* primes, long long N, int S) {
+    const long long threads = S == 1 ? (N + 1) / 2 : N;
+    const dim3 g((unsigned)((threads + 255) / 256), (unsigned)gm.ne);
+    if (S == 1) k_gadget_mac1<NC><<<g, 256, 0, stream()>>>(gm, D, primes, N);
+    else k_gadget_mac<NC><<<g, 256, 0, stream()>>>(gm, D, primes, N, S);
+    note_launch();
+    return (int)cudaGetLastError();
+}
+
+// Whether gadget_mac_all takes these operands: one pool, FP64 primes, every key polynomial
+// active at the same extended limbs, blocks apart from one another and the digits.
+bool gadget_all_ok(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly) {
+    IncNtt* t = pool(out);
+    const uint64_t ext = ksk[0]->b->rns_mask, mask = poly->pub.rns_mask;
+    const int nd = popcount64(mask), comps = (int)out->r + 1;
+    if (nd == 0 || comps > kGadgetComps || comps < 2 || nd * comps > kGadgetKeys || t->pub.l > 64) return false;
+    auto covers = [&](Poly* p, uint64_t m) {
+        return p && p->base && pool_of(p) == t && (p->pub.allocated_l >= 64 || (m >> p->pub.allocated_l) == 0);
+    };
+    if (!covers(poly, mask) || (t->pub.l < 64 && (ext >> t->pub.l) != 0)) return false;
+    uint32_t idx[64];
+    const int ne = mask_indices(ext, t->pub.l, idx);
+    for (int i = 0; i < ne; ++i)
+        if (!t->info[idx[i]].fp64) return false;
+    if (ne == 0 || t->logP < 8 || t->logP > 17) return false;
+    for (int c = 0; c < comps; ++c) {
+        Poly* o = P_(c < (int)out->r ? out->a[c] : out->b);
+        if (!covers(o, ext) || o == poly) return false;
+        for (int j = 0; j < nd; ++j) {
+            RNS_MLWE k = ksk[j];
+            if (!k || (int)k->r + 1 != comps) return false;
+            Poly* kp = P_(c < (int)k->r ? k->a[c] : k->b);
+            if (!covers(kp, ext) || kp->pub.rns_mask != ext || kp == o) return false;
+        }
+    }
+    return true;
+}
+
+// Digit polynomials of `poly` times the keys into out's extended limbs (mode as GadgetMac).
+void gadget_mac_all(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly, int mode, const char* where) {
+    IncNtt* t = pool(out);
+    const long long N = (long long)t->pub.N;
+    const uint64_t ext = ksk[0]->b->rns_mask;
+    const int comps = (int)out->r + 1;
+    uint32_t dig[64];
+    GadgetMac gm;
+    memset(&gm, 0, sizeof gm);
+    const int nd = mask_indices(poly->pub.rns_mask, t->pub.l, dig);
+    gm.ne = mask_indices(ext, t->pub.l, gm.prime);
+    for (int c = 0; c < comps; ++c) gm.out[c] = P_(c < (int)out->r ? out->a[c] : out->b)->base;
+    int per = (int)(kGadgetScratch / ((size_t)gm.ne * N * 8));
+    if (per < 1) per = 1;
+    if (per > nd) per = nd;
+    uint64_t* D = (uint64_t*)device_alloc((size_t)per * gm.ne * N * 8);
+    if (!D) return;
+    for (int j0 = 0; j0 < nd;) {
+        // consecutive limbs are rows N apart
+        int n = 1;
+        while (j0 + n < nd && n < per && dig[j0 + n] == dig[j0] + (uint32_t)n) ++n;
+        RowSet rs;
+        memset(&rs, 0, sizeof rs);
+        for (int i = 0; i < gm.ne; ++i) {
+            rs.in[i] = poly->pub.coeffs[dig[j0]];
+            rs.out[i] = D + (long long)i * N;
+            rs.prime[i] = gm.prime[i];
+        }
+        rs.nlimbs = gm.ne;
+        rs.split = (int)t->pub.split_degree;
+        rs.logP = t->logP;
+        rs.batch = 1;
+        rs.reduce_input = 1;
+        rs.digits = n;
+        rs.digit_in_stride = N;
+        rs.digit_stride = (long long)gm.ne * N;
+        mark_fp64(rs, t);
+        if (!ntt_f64_eligible(rs)) {  // the integer transforms were asked for: digit by digit
+            for (int d = 0; d < n; ++d) {
+                RowSet one = rs;
+                one.digits = 0;
+                one.digit_in_stride = one.digit_stride = 0;
+                for (int i = 0; i < gm.ne; ++i) {
+                    one.in[i] = poly->pub.coeffs[dig[j0 + d]];
+                    one.out[i] = rs.out[i] + d * rs.digit_stride;
+                }
+                if (!check_cuda(launch_ntt(one, t->d_info, false, stream()), where)) return;
+            }
+        } else if (!check_cuda(launch_ntt(rs, t->d_info, false, stream()), where)) {
+            return;
+        }
+        for (int d = 0; d < n; ++d)
+            for (int c = 0; c < comps; ++c) {
+                RNS_MLWE k = ksk[j0 + d];
+                gm.key[d * comps + c] = P_(c < (int)k->r ? k->a[c] : k->b)->base;
+            }
+        gm.digits = n;
+        gm.mode = mode;
+        const int S = (int)t->pub.split_degree;
+        const int e = comps == 2   ? launch_gadget_mac<2>(gm, D, t->d_info, N, S)
+                      : comps == 3 ? launch_gadget_mac<3>(gm, D, t->d_info, N, S)
+                                   : launch_gadget_mac<4>(gm, D, t->d_info, N, S);
+        if (!check_cuda(e, where)) return;
+        if (mode == 0) mode = 1;
+        if (mode == 3) mode = 2;
+        j0 += n;
+    }
+    set_masks(out, ext);
+    device_free(D);
+}
+
 
 // Gaussian integers (truncated Box-Muller draws), four per ChaCha20 block from ctr on.
 __global__ void k_gauss_int(int64_t* out, long long n, double sigma, const __grid_constant__ PrngKey key,
@@ -455,6 +734,10 @@ void mlwe_RNSc_to_RNS(void* out, void* in) {
     RNS_MLWE o = as_mlwe(out), i = as_mlwe(in);
     prefetch_mlwe(i);
     prefetch_mlwe(o);
+    if (transform_together(o, i, false, vc_where_)) {
+        VC_FINISH();
+        return;
+    }
     for (uint64_t k = 0; k < o->r; ++k) polynomial_RNSc_to_RNS(o->a[k], i->a[k]);
     polynomial_RNSc_to_RNS(o->b, i->b);
     VC_FINISH();
@@ -463,6 +746,10 @@ void mlwe_RNSc_to_RNS(void* out, void* in) {
 void mlwe_RNS_to_RNSc(void* out, void* in) {
     VC_ENTER("mlwe_RNS_to_RNSc");
     RNS_MLWE o = as_mlwe(out), i = as_mlwe(in);
+    if (transform_together(o, i, true, vc_where_)) {
+        VC_FINISH();
+        return;
+    }
     for (uint64_t k = 0; k < o->r; ++k) polynomial_RNS_to_RNSc(o->a[k], i->a[k]);
     polynomial_RNS_to_RNSc(o->b, i->b);
     VC_FINISH();
@@ -645,8 +932,9 @@ void mlwe_round_division_RNSc(void* out, uint64_t divide_mask) {
     VC_ENTER("mlwe_round_division_RNSc");
     if (divide_mask == 0) return;
     RNS_MLWE o = as_mlwe(out);
-    for (uint64_t k = 0; k < o->r; ++k) polynomial_round_division_RNSc_wo_free(o->a[k], divide_mask);
-    polynomial_round_division_RNSc_wo_free(o->b, divide_mask);
+    std::vector<Poly*> comps(o->r + 1);
+    for (uint64_t k = 0; k <= o->r; ++k) comps[k] = P_(k < o->r ? o->a[k] : o->b);
+    op_round_divide(comps.data(), (int)comps.size(), divide_mask, vc_where_);
     VC_FINISH();
 }
 
@@ -699,8 +987,15 @@ void mlwe_RNSc_GHS_hybrid_keyswitch(void* out, void* in, void* ksk, uint64_t lvl
     const uint64_t extended = K[c0][0]->b->rns_mask;
     const uint64_t divide_mask = extended & ~i->b->rns_mask;
     set_masks(o, extended);
-    zero_mlwe(o, vc_where_);
-    for (uint64_t k = 0; k < i->r; ++k)
+    uint64_t first = c0;
+    if (gadget_all_ok(o, K[c0], P_(i->a[c0]))) {  // writes every extended row: only the others are zeroed
+        zero_mlwe(o, vc_where_, ~extended);
+        gadget_mac_all(o, K[c0], P_(i->a[c0]), 3, vc_where_);
+        first = c0 + 1;
+    } else {
+        zero_mlwe(o, vc_where_);
+    }
+    for (uint64_t k = first; k < i->r; ++k)
         if (K[k] != nullptr) gadget_mac(o, K[k], P_(i->a[k]), 2, vc_where_);
     mlwe_RNS_to_RNSc(o, o);
     mlwe_round_division_RNSc(o, divide_mask);
@@ -828,8 +1123,15 @@ void mgsw_external_product(void* out, void* mgsw, void* in, uint64_t ell, uint64
     const uint64_t r = i->r;
     const uint64_t extended = G[0]->b->rns_mask;
     set_masks(o, extended);
-    zero_mlwe(o, vc_where_);
-    for (uint64_t j = 0; j < r; ++j) gadget_mac(o, &G[j * ell], P_(i->a[j]), 1, vc_where_);
+    uint64_t first = 0;
+    if (r > 0 && o != i && gadget_all_ok(o, G, P_(i->a[0]))) {
+        zero_mlwe(o, vc_where_, ~extended);
+        gadget_mac_all(o, G, P_(i->a[0]), 0, vc_where_);
+        first = 1;
+    } else {
+        zero_mlwe(o, vc_where_);
+    }
+    for (uint64_t j = first; j < r; ++j) gadget_mac(o, &G[j * ell], P_(i->a[j]), 1, vc_where_);
     gadget_mac(o, &G[r * ell], P_(i->b), 1, vc_where_);
     if (special_primes > 0) {
         mlwe_RNS_to_RNSc(o, o);

@@ -186,11 +186,13 @@ int launch_permute(const EwSet& set, uint64_t N, int split, uint64_t gen, const 
 int launch_mul_xai(const EwSet& set, uint64_t N, uint64_t a, bool minus1, const PrimeInfo* d_primes,
                    cudaStream_t st);
 
-// Rounded (round=true) or floored division by the prime of limb `drop`, applied to
-// the limbs listed in `set` (rns_polynomial.c:905-976).  set.a[k] must be the
-// dropped limb's row for every k; set.out[k] the limb rows to update.
+// Rounded or floored division by one prime of `polys` polynomials with the same active
+// limbs (rns_polynomial.c:905-976): set.out holds the limb rows to update, polynomial by
+// polynomial, drop_row each polynomial's dropped limb.
+constexpr int kDividePolys = 4;
 struct DivideArgs {
-    uint64_t* drop_row;
+    uint64_t* drop_row[kDividePolys];
+    int polys;
     uint64_t half_drop;      // floor(p/2) (0 for floor division)
     uint64_t p;              // dropped prime
     uint32_t drop_prime;     // its pool index

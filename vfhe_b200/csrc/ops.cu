@@ -149,21 +149,28 @@ __global__ void k_mul_xai(const __grid_constant__ EwSet set, const PrimeInfo* __
 }
 
 // One prime dropped: t = (c_p + half) mod p; c_i <- (c_i + half - t) * p^-1 mod q_i; c_p <- 0.
-__global__ void k_divide(const __grid_constant__ EwSet set, DivideArgs d, const PrimeInfo* __restrict__ primes,
-                         long long n) {
-    for (long long x = blockIdx.x * (long long)blockDim.x + threadIdx.x; x < n;
-         x += (long long)gridDim.x * blockDim.x) {
-        const uint64_t cp = d.drop_row[x];
-        const uint64_t t = add_mod(cp, d.half_drop, d.p);
-        for (int k = 0; k < set.nlimbs; ++k) {
-            const PrimeInfo& pi = primes[set.prime[k]];
-            const uint64_t q = pi.q;
-            uint64_t c = set.out[k][x];
-            c = add_mod(c, reduce64(d.half_drop, pi), q);
-            c = sub_mod(c, reduce64(t, pi), q);
-            set.out[k][x] = shoup(c, set.s[k], set.s_sh[k], q);
+// Polynomial blockIdx.y's limbs are slots [y per, (y + 1) per).  A block takes 64 coefficients
+// and deals the limbs to four rows of threads: one thread per coefficient walking every limb
+// left most of the GPU idle (10 limbs at N = 2^14: 8.9 us against 4).
+__global__ void __launch_bounds__(256) k_divide(const __grid_constant__ EwSet set, const __grid_constant__ DivideArgs d,
+                                                const PrimeInfo* __restrict__ primes, int per, long long n) {
+    uint64_t* drop = d.drop_row[blockIdx.y];
+    for (long long base = blockIdx.x * 64LL; base < n; base += gridDim.x * 64LL) {
+        const long long x = base + threadIdx.x;
+        if (x < n) {
+            const uint64_t t = add_mod(drop[x], d.half_drop, d.p);
+            for (int j = threadIdx.y; j < per; j += 4) {
+                const int k = blockIdx.y * per + j;
+                const PrimeInfo& pi = primes[set.prime[k]];
+                const uint64_t q = pi.q;
+                uint64_t c = set.out[k][x];
+                c = add_mod(c, reduce64(d.half_drop, pi), q);
+                c = sub_mod(c, reduce64(t, pi), q);
+                set.out[k][x] = shoup(c, set.s[k], set.s_sh[k], q);
+            }
         }
-        d.drop_row[x] = 0;
+        __syncthreads();  // every limb has read the dropped row
+        if (x < n && threadIdx.y == 0) drop[x] = 0;
     }
 }
 
@@ -292,10 +299,11 @@ int launch_mul_xai(const EwSet& set, uint64_t N, uint64_t a, bool minus1, const 
 }
 
 int launch_divide(const EwSet& set, const DivideArgs& d, const PrimeInfo* d_primes, cudaStream_t st) {
-    long long blocks = (set.n + kThreads - 1) / kThreads;
+    long long blocks = (set.n + 63) / 64;
     if (blocks > 4096) blocks = 4096;
     if (blocks < 1) blocks = 1;
-    k_divide<<<(unsigned)blocks, kThreads, 0, st>>>(set, d, d_primes, set.n);
+    k_divide<<<dim3((unsigned)blocks, (unsigned)d.polys), dim3(64, 4), 0, st>>>(set, d, d_primes, set.nlimbs / d.polys,
+                                                                              set.n);
     return (int)cudaGetLastError();
 }
 
