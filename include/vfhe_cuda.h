@@ -291,6 +291,13 @@ int vfhe_cuda_synchronize(void);
 /* Number of transform and batched-CKKS kernels this engine has launched so far. */
 uint64_t vfhe_cuda_launch_count(void);
 
+/* Copy `count` residue rows of an RNS_Polynomial (pool rows rows[0..count)) into host
+ * memory, h_out [count][N].  The same values as reading coeffs[rows[k]] from the host, by
+ * copies that leave the rows' pages on the device: a direct read moves them to the host
+ * page by page, and the next kernel that uses them moves them back.  Returns 0 on success.
+ * No counterpart in the reference (its rows are host memory). */
+int vfhe_cuda_poly_read_rows(void *poly, uint64_t *h_out, const uint32_t *rows, uint32_t count);
+
 /* Batched negacyclic (incomplete) NTT over a device buffer laid out as
  * [batch][nlimbs][N] uint64 residues; limb slot k uses pool prime limbs[k] of the
  * incNTT `ntt` (same split_degree layout as polynomial_RNSc_to_RNS).

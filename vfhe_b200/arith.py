@@ -454,9 +454,20 @@ class Polynomial:
         return out
 
     # -- coefficient IO
-    def rows(self) -> np.ndarray:
-        """Raw rows of the ring's limbs, [ell][N] uint64, in the engine's row layout."""
-        return np.stack([self.row(i).copy() for i in self.ring.prime_indices])
+    def rows(self, out: np.ndarray | None = None) -> np.ndarray:
+        """Raw rows of the ring's limbs, [ell][N] uint64, in the engine's row layout (into
+        ``out``, contiguous, when given)."""
+        eng, idx = self.ring.engine, self.ring.prime_indices
+        if out is None:
+            out = np.empty((len(idx), self.ring.N), dtype=np.uint64)
+        if eng.name == "cuda":
+            self._lib.vfhe_cuda_poly_read_rows(self.obj, self.ring.ffi.from_buffer("uint64_t[]", out),
+                                               self.ring.ffi.new("uint32_t[]", idx), len(idx))
+            self._chk("vfhe_cuda_poly_read_rows")
+        else:
+            for k, i in enumerate(idx):
+                out[k] = self.row(i)
+        return out
 
     def set_rows(self, rows: np.ndarray) -> None:
         for k, idx in enumerate(self.ring.prime_indices):

@@ -351,7 +351,10 @@ def bootstrap_key_tensor(bk) -> torch.Tensor:
 
 def ciphertext_rows(ct: MLWE) -> np.ndarray:
     """[2][L][N] raw rows of a rank-1 ciphertext."""
-    return np.stack([ct.component_rows(0), ct.component_rows(1)])
+    out = np.empty((2, ct.ring.ell, ct.ring.N), dtype=np.uint64)
+    for i in range(2):
+        ct.component_rows(i, out[i])
+    return out
 
 
 def key_tensor(ks: MLWE_Set, component: int = 0) -> torch.Tensor:

@@ -115,7 +115,7 @@ int* flag() {
 void ew_mask(EwOp op, Poly* out, Poly* a, Poly* b, uint64_t mask, const char* where) {
     prefetch_poly(a);
     prefetch_poly(b);
-    prefetch_poly(out);
+    prefetch_out(out);
     EwSet s = poly_set(out, a, b, mask);
     check_cuda(launch_ew(op, s, pool_of(out)->d_info, stream()), where);
 }
@@ -131,7 +131,7 @@ int int_array_to_RNS_device(void* out, const int64_t* d_in, cudaStream_t st) {
     Poly* o = as_poly(out);
     IncNtt* t = pool_of(o);
     const uint64_t N = t->pub.N;
-    prefetch_poly(o);
+    prefetch_out(o);
     EwSet s = poly_set(o, nullptr, nullptr, o->pub.rns_mask);
     for (int k = 0; k < s.nlimbs; ++k) s.a[k] = (const uint64_t*)d_in;
     int ls = 0;
@@ -227,7 +227,7 @@ void array_to_RNS(void* out, uint64_t** in) {
         VC_CHECK(cudaMemcpyAsync(d_in + k * N, row, N * 8, cudaMemcpyHostToDevice, stream()));
         s.a[k] = d_in + k * N;
     }
-    prefetch_poly(o);
+    prefetch_out(o);
     int ls = 0;
     while ((1ULL << ls) < t->pub.split_degree) ++ls;
     if (s.nlimbs) {
@@ -244,7 +244,7 @@ void polynomial_gen_random_RNSc_polynomial(void* out) {
     VC_ENTER("polynomial_gen_random_RNSc_polynomial");
     if (!valid_poly(out, vc_where_)) return;
     Poly* o = as_poly(out);
-    prefetch_poly(o);
+    prefetch_out(o);
     EwSet s = poly_set(o, nullptr, nullptr, o->pub.rns_mask);
     const uint64_t ctr = prng_advance((uint64_t)((s.n + 3) / 4) * (uint64_t)(s.nlimbs ? s.nlimbs : 1));
     VC_CHECK(launch_sample_uniform(s, prng_key(), ctr, pool_of(o)->d_info, stream()));
@@ -255,7 +255,7 @@ void polynomial_gen_gaussian_RNSc_polynomial(void* out, double sigma) {
     VC_ENTER("polynomial_gen_gaussian_RNSc_polynomial");
     if (!valid_poly(out, vc_where_)) return;
     Poly* o = as_poly(out);
-    prefetch_poly(o);
+    prefetch_out(o);
     EwSet s = poly_set(o, nullptr, nullptr, o->pub.rns_mask);
     const uint64_t ctr = prng_advance((uint64_t)((s.n + 3) / 4));
     VC_CHECK(launch_sample_gaussian(s, sigma, prng_key(), ctr, pool_of(o)->d_info, stream()));
@@ -273,7 +273,7 @@ static void product(void* out, void* in1, void* in2, int mode, bool set_mask_onl
     o->pub.rns_mask = mask;
     prefetch_poly(a);
     prefetch_poly(b);
-    prefetch_poly(o);
+    prefetch_out(o);
     EwSet s = poly_set(o, a, b, mask);
     check_cuda(launch_inc_product(mode, s, (int)t->pub.split_degree, t->logP, t->d_info, stream()), where);
 }
@@ -297,7 +297,7 @@ void polynomial_multo_RNS_polynomial(void* out, void* in) {
     const uint64_t mask = o->pub.rns_mask & i->pub.rns_mask;
     o->pub.rns_mask = mask;
     IncNtt* t = pool_of(o);
-    prefetch_poly(o);
+    prefetch_out(o);
     prefetch_poly(i);
     EwSet s = poly_set(o, i, o, mask);
     VC_CHECK(launch_inc_product(0, s, (int)t->pub.split_degree, t->logP, t->d_info, stream()));
@@ -336,7 +336,7 @@ static void scale_by(Poly* o, Poly* a, const uint64_t* per_limb, uint64_t unifor
     const uint64_t mask = a->pub.rns_mask;
     o->pub.rns_mask = mask;
     prefetch_poly(a);
-    prefetch_poly(o);
+    prefetch_out(o);
     EwSet s = poly_set(o, a, nullptr, mask);
     for (int k = 0; k < s.nlimbs; ++k) {
         const uint64_t q = t->info[s.prime[k]].q;
@@ -378,7 +378,7 @@ static void add_integer(Poly* o, Poly* a, uint64_t in2, long long count, const c
     const uint64_t mask = a->pub.rns_mask;
     o->pub.rns_mask = mask;
     if (o != a) ew_mask(EW_COPY, o, a, nullptr, mask, where);
-    prefetch_poly(o);
+    prefetch_out(o);
     EwSet s = poly_set(o, o, nullptr, mask);
     s.n = count;
     for (int k = 0; k < s.nlimbs; ++k) s.s[k] = host_reduce_signed(in2, t->info[s.prime[k]].q);
@@ -430,7 +430,7 @@ void polynomial_RNSc_to_RNS(void* out, void* in) {
     Poly* i = as_poly(in);
     o->pub.rns_mask = i->pub.rns_mask;
     prefetch_poly(i);
-    prefetch_poly(o);
+    prefetch_out(o);
     VC_CHECK(poly_ntt(o, i, o->pub.rns_mask, false));
     VC_FINISH();
 }
@@ -442,7 +442,7 @@ void polynomial_RNS_to_RNSc(void* out, void* in) {
     Poly* i = as_poly(in);
     o->pub.rns_mask = i->pub.rns_mask;
     prefetch_poly(i);
-    prefetch_poly(o);
+    prefetch_out(o);
     VC_CHECK(poly_ntt(o, i, o->pub.rns_mask, true));
     VC_FINISH();
 }
@@ -465,7 +465,7 @@ void polynomial_RNSc_mod_reduce_lifted(void* out, void* in, uint64_t idx) {
         return;
     }
     prefetch_poly(i);
-    prefetch_poly(o);
+    prefetch_out(o);
     EwSet s = poly_set(o, nullptr, nullptr, o->pub.rns_mask);
     for (int k = 0; k < s.nlimbs; ++k) s.a[k] = i->pub.coeffs[idx];
     VC_CHECK(launch_ew(EW_REDUCE, s, pool_of(o)->d_info, stream()));
@@ -588,7 +588,7 @@ int polynomial_RNS_inverse(void* out, void* in) {
     if (!f) return -1;
     *f = 0;
     prefetch_poly(i);
-    prefetch_poly(o);
+    prefetch_out(o);
     EwSet s = poly_set(o, i, nullptr, i->pub.rns_mask);
     if (s.nlimbs) {
         k_inverse<<<grid_for(s.n, s.nlimbs), 256, 0, stream()>>>(s, t->d_info, f);
@@ -640,7 +640,7 @@ static void slots(void* out, void* in, int mode, long long a0, long long a1, con
     if (mode == 1) a0 %= (long long)t->P;
     o->pub.rns_mask = i->pub.rns_mask;
     prefetch_poly(i);
-    prefetch_poly(o);
+    prefetch_out(o);
     EwSet s = poly_set(o, i, nullptr, i->pub.rns_mask);
     if (!s.nlimbs) return;
     const long long total = mode == 2 ? (long long)t->pub.split_degree : (long long)t->pub.N;
@@ -682,6 +682,32 @@ void polynomial_RNS_copy_slot(void* out, uint64_t dst, void* in, uint64_t src) {
     if (!valid_poly(out, vc_where_) || !valid_poly(in, vc_where_)) return;
     slots(out, in, 2, (long long)dst, (long long)src, vc_where_);
     VC_FINISH();
+}
+
+int vfhe_cuda_poly_read_rows(void* poly, uint64_t* h_out, const uint32_t* rows, uint32_t count) {
+    VC_ENTER_RET("vfhe_cuda_poly_read_rows", 1);
+    if (!valid_poly(poly, vc_where_)) return 1;
+    Poly* p = as_poly(poly);
+    const uint64_t N = p->pub.ntt->N;
+    if (count && (!h_out || !rows || !p->base)) {
+        set_error(vc_where_, "null buffer, row list or rows");
+        return 1;
+    }
+    for (uint32_t k = 0; k < count; ++k)
+        if (rows[k] >= p->pub.allocated_l) {
+            set_error(vc_where_, "row outside the polynomial");
+            return 1;
+        }
+    // runs of neighbouring rows in one copy each
+    for (uint32_t k = 0; k < count;) {
+        uint32_t n = 1;
+        while (k + n < count && rows[k + n] == rows[k] + n) ++n;
+        if (!VC_CHECK(cudaMemcpyAsync(h_out + (uint64_t)k * N, p->base + (uint64_t)rows[k] * N, n * N * sizeof(uint64_t),
+                                      cudaMemcpyDefault, stream())))
+            return 1;
+        k += n;
+    }
+    return vc::sync(vc_where_) ? 0 : 1;
 }
 
 void polynomial_RNS_get_hash(uint64_t* out, void* p) {

@@ -20,10 +20,27 @@ inline int mask_indices(uint64_t mask, uint64_t l, uint32_t* idx) {
 inline IncNtt* pool_of(Poly* p) { return reinterpret_cast<IncNtt*>(p->pub.ntt); }
 
 inline int& call_depth();
-inline void prefetch_poly(Poly* p) {
-    if (call_depth() > 1) return;  // the outermost call already prefetched its operands
-    if (p && p->base) prefetch_to_device(p->base, sizeof(uint64_t) * p->pub.allocated_l * p->pub.ntt->N);
+
+// Operands of 2 MiB or more are prefetched to the device (prefetch_to_device), which costs
+// 70-85 us of driver time even when the pages are there.  A polynomial below 8 MiB is
+// therefore prefetched once: when the first kernel reads it (the host may have written it),
+// or writes it in a new block (a freed polynomial's block is on the device already, where
+// kernels left it).  After that its pages move only if the host touches them, and the faults
+// of that case cost 50-175 us up to 4 MB.  From 8 MiB on they cost a millisecond and more, so
+// those are prefetched at every use.  One product of 2.5 MB polynomials: 12 prefetches, 960
+// us, before; none once its operands have been used.
+constexpr size_t kPrefetchEveryUse = 8ULL << 20;
+
+inline void prefetch_use(Poly* p, bool written) {
+    if (!p || !p->base) return;
+    const size_t bytes = sizeof(uint64_t) * p->pub.allocated_l * p->pub.ntt->N;
+    // in a nested call the outermost one already prefetched its operands
+    if (call_depth() <= 1 && (bytes >= kPrefetchEveryUse || !(p->on_device || (written && p->recycled))))
+        prefetch_to_device(p->base, bytes);
+    p->on_device = true;
 }
+inline void prefetch_poly(Poly* p) { prefetch_use(p, false); }
+inline void prefetch_out(Poly* p) { prefetch_use(p, true); }
 
 inline EwSet empty_set(long long n) {
     EwSet s;

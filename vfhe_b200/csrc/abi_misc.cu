@@ -129,7 +129,7 @@ void polynomial_base_conversion_RNSc(void* out, void* in, void* params) {
     if (o != i) {
         EwSet s = poly_set(o, i, nullptr, in_mask & out_mask);
         prefetch_poly(i);
-        prefetch_poly(o);
+        prefetch_out(o);
         VC_CHECK(launch_ew(EW_COPY, s, pool_of(o)->d_info, stream()));
     }
     BaseConv* bc = (BaseConv*)params;

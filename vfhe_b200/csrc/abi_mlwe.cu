@@ -39,10 +39,10 @@ void del_mlwe(RNS_MLWE m) {
 inline Poly* P_(RNS_Polynomial p) { return reinterpret_cast<Poly*>(p); }
 inline IncNtt* pool(RNS_MLWE m) { return reinterpret_cast<IncNtt*>(m->b->ntt); }
 
-void prefetch_mlwe(RNS_MLWE m) {
+void prefetch_mlwe(RNS_MLWE m, bool written = false) {
     if (!m) return;
-    for (uint64_t i = 0; i < m->r; ++i) prefetch_poly(P_(m->a[i]));
-    prefetch_poly(P_(m->b));
+    for (uint64_t i = 0; i < m->r; ++i) prefetch_use(P_(m->a[i]), written);
+    prefetch_use(P_(m->b), written);
 }
 
 void set_masks(RNS_MLWE m, uint64_t mask);
@@ -99,6 +99,7 @@ bool transform_together(RNS_MLWE o, RNS_MLWE i, bool inverse, const char* where)
     rs.batch = 1;
     mark_fp64(rs, t);
     if (!check_cuda(launch_ntt(rs, t->d_info, inverse, stream()), where)) return true;
+    for (uint64_t c = 0; c <= o->r; ++c) P_(c < o->r ? o->a[c] : o->b)->on_device = true;
     set_masks(o, mask);
     return true;
 }
@@ -295,7 +296,11 @@ void gadget_mac_all(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly, int mode, const cha
     memset(&gm, 0, sizeof gm);
     const int nd = mask_indices(poly->pub.rns_mask, t->pub.l, dig);
     gm.ne = mask_indices(ext, t->pub.l, gm.prime);
-    for (int c = 0; c < comps; ++c) gm.out[c] = P_(c < (int)out->r ? out->a[c] : out->b)->base;
+    for (int c = 0; c < comps; ++c) {
+        Poly* o = P_(c < (int)out->r ? out->a[c] : out->b);
+        o->on_device = true;
+        gm.out[c] = o->base;
+    }
     int per = (int)(kGadgetScratch / ((size_t)gm.ne * N * 8));
     if (per < 1) per = 1;
     if (per > nd) per = nd;
@@ -733,7 +738,7 @@ void mlwe_RNSc_to_RNS(void* out, void* in) {
     VC_ENTER("mlwe_RNSc_to_RNS");
     RNS_MLWE o = as_mlwe(out), i = as_mlwe(in);
     prefetch_mlwe(i);
-    prefetch_mlwe(o);
+    prefetch_mlwe(o, true);
     if (transform_together(o, i, false, vc_where_)) {
         VC_FINISH();
         return;
@@ -883,7 +888,7 @@ static void xai(Poly* o, Poly* i, uint64_t a, bool minus1, const char* where) {
         return;
     }
     prefetch_poly(i);
-    prefetch_poly(o);
+    prefetch_out(o);
     EwSet s = poly_set(o, i, nullptr, i->pub.rns_mask);
     check_cuda(launch_mul_xai(s, N, a, minus1, t->d_info, stream()), where);
 }

@@ -46,7 +46,7 @@ bool sync(const char* where);
 
 // ---------------------------------------------------------------- memory
 // Managed (host+device addressable) blocks from a size-bucketed cache.
-void* managed_alloc(size_t bytes);
+void* managed_alloc(size_t bytes, bool* recycled = nullptr);  // recycled: a block freed before, not a new one
 void managed_free(void* p);
 // Device-only scratch from a size-bucketed cache.
 void* device_alloc(size_t bytes);
@@ -69,6 +69,8 @@ struct IncNtt {
 struct Poly {
     _RNS_Polynomial pub;  // public prefix; must stay first
     uint64_t* base = nullptr;  // managed block, allocated_l * N residues
+    bool on_device = false;    // a kernel has used the block since the polynomial was made
+    bool recycled = false;     // the block belonged to a freed polynomial before
 };
 
 struct Mlwe {

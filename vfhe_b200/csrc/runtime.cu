@@ -98,7 +98,7 @@ size_t round_bytes(size_t b) {
     size_t step = p >> 3;
     return (b + step - 1) / step * step;
 }
-void* cache_alloc(Cache& c, size_t bytes, bool managed) {
+void* cache_alloc(Cache& c, size_t bytes, bool managed, bool* recycled = nullptr) {
     size_t rb = round_bytes(bytes);
     {
         std::lock_guard<std::mutex> lk(c.mu);
@@ -106,6 +106,7 @@ void* cache_alloc(Cache& c, size_t bytes, bool managed) {
         if (it != c.free_blocks.end()) {
             void* p = it->second;
             c.free_blocks.erase(it);
+            if (recycled) *recycled = true;
             return p;
         }
     }
@@ -128,9 +129,10 @@ void cache_free(Cache& c, void* p) {
 }
 }  // namespace
 
-void* managed_alloc(size_t bytes) {
+void* managed_alloc(size_t bytes, bool* recycled) {
+    if (recycled) *recycled = false;
     if (!ensure_ready()) return nullptr;
-    return cache_alloc(managed_cache(), bytes, true);
+    return cache_alloc(managed_cache(), bytes, true, recycled);
 }
 void managed_free(void* p) { cache_free(managed_cache(), p); }
 void* device_alloc(size_t bytes) {
@@ -512,7 +514,7 @@ Poly* poly_create(uint64_t N, uint64_t mask, IncNtt* t) {
     }
     Poly* p = new Poly();
     const uint64_t l = t->pub.l;
-    p->base = (uint64_t*)managed_alloc(sizeof(uint64_t) * l * t->pub.N);
+    p->base = (uint64_t*)managed_alloc(sizeof(uint64_t) * l * t->pub.N, &p->recycled);
     p->pub.coeffs = (uint64_t**)malloc(sizeof(uint64_t*) * (l ? l : 1));
     for (uint64_t i = 0; i < l; ++i) p->pub.coeffs[i] = p->base ? p->base + i * t->pub.N : nullptr;
     p->pub.ntt = &t->pub;

@@ -390,8 +390,8 @@ class MLWE:
         v.set_rows(rows)
         v.rns_mask = self.ring.mask
 
-    def component_rows(self, i: int) -> np.ndarray:
-        return self.component(i).rows()
+    def component_rows(self, i: int, out: np.ndarray | None = None) -> np.ndarray:
+        return self.component(i).rows(out)
 
     def obj_a_i(self, j: int):
         return self.ring.ffi.cast("RNS_MLWE", self.obj).a[j]
