@@ -79,7 +79,9 @@ __device__ __forceinline__ void mac_slot(uint64_t* oa, uint64_t* ob, const uint6
 
 // mac_slot for all S output blocks of slot x at once (S = 2 or 4): every digit's S
 // blocks of D and of both key components are loaded once (3 S loads per digit for S
-// outputs, the traffic of a pointwise product).  Same exact FP64 arithmetic and result.
+// outputs, the traffic of a pointwise product), a digit ahead of their products: with 16
+// warps an SM the loads' latency bound the work list's multiply-accumulates (64 uneven jobs
+// 3.18 -> 3.13 ms).  Same exact FP64 arithmetic and result.
 template <int S>
 __device__ __forceinline__ void mac_slots(uint64_t* oa, uint64_t* ob, const uint64_t* d, long long dstr,
                                           const uint64_t* ka, const uint64_t* kb, long long kstr, int nd, long long P,
@@ -88,16 +90,31 @@ __device__ __forceinline__ void mac_slots(uint64_t* oa, uint64_t* ob, const uint
     double sa[S], sb[S], wa[S], wb[S];
 #pragma unroll
     for (int o = 0; o < S; ++o) sa[o] = sb[o] = wa[o] = wb[o] = 0.0;
+    uint64_t rv[S], ra[S], rb[S];  // the next digit's operands, loaded a digit ahead
+#pragma unroll
+    for (int i = 0; i < S; ++i) {
+        rv[i] = d[(long long)i * P + x];
+        ra[i] = ka[(long long)i * P + x];
+        rb[i] = kb[(long long)i * P + x];
+    }
     int terms = 0;
     for (int j = 0; j < nd; ++j) {
-        double v[S], ya[S], yqa[S], yb[S], yqb[S];
+        // the digit is the multiplier of both key products (one quotient for two)
+        double v[S], vq[S], ya[S], yb[S];
 #pragma unroll
         for (int i = 0; i < S; ++i) {
-            v[i] = f_from_u64(d[j * dstr + (long long)i * P + x]);
-            ya[i] = f_from_u64(ka[j * kstr + (long long)i * P + x]);
-            yb[i] = f_from_u64(kb[j * kstr + (long long)i * P + x]);
-            yqa[i] = __dmul_rn(ya[i], qinv);
-            yqb[i] = __dmul_rn(yb[i], qinv);
+            v[i] = f_from_u64(rv[i]);
+            vq[i] = __dmul_rn(v[i], qinv);
+            ya[i] = f_from_u64(ra[i]);
+            yb[i] = f_from_u64(rb[i]);
+        }
+        if (j + 1 < nd) {
+#pragma unroll
+            for (int i = 0; i < S; ++i) {
+                rv[i] = d[(j + 1) * dstr + (long long)i * P + x];
+                ra[i] = ka[(j + 1) * kstr + (long long)i * P + x];
+                rb[i] = kb[(j + 1) * kstr + (long long)i * P + x];
+            }
         }
 #pragma unroll
         for (int o = 0; o < S; ++o)
@@ -105,8 +122,8 @@ __device__ __forceinline__ void mac_slots(uint64_t* oa, uint64_t* ob, const uint
             for (int i = 0; i < S; ++i) {
                 const int k = o - i;
                 const int kk = k < 0 ? k + S : k;
-                const double ta = f_mulmod(v[i], ya[kk], yqa[kk], q);
-                const double tb = f_mulmod(v[i], yb[kk], yqb[kk], q);
+                const double ta = f_mulmod(ya[kk], v[i], vq[i], q);
+                const double tb = f_mulmod(yb[kk], v[i], vq[i], q);
                 if (k < 0) {
                     wa[o] = __dadd_rn(wa[o], ta);
                     wb[o] = __dadd_rn(wb[o], tb);
@@ -133,10 +150,10 @@ __device__ __forceinline__ void mac_slots(uint64_t* oa, uint64_t* ob, const uint
     const double wq = __dmul_rn(w, qinv);
 #pragma unroll
     for (int o = 0; o < S; ++o) {
-        const double ra = __dadd_rn(sa[o], f_mulmod(wa[o], w, wq, q));
-        const double rb = __dadd_rn(sb[o], f_mulmod(wb[o], w, wq, q));
-        oa[(long long)o * P + x] = f_to_canonical(-ra, q, qinv, pi.q);
-        ob[(long long)o * P + x] = f_to_canonical(-rb, q, qinv, pi.q);
+        const double za = __dadd_rn(sa[o], f_mulmod(wa[o], w, wq, q));
+        const double zb = __dadd_rn(sb[o], f_mulmod(wb[o], w, wq, q));
+        oa[(long long)o * P + x] = f_to_canonical(-za, q, qinv, pi.q);
+        ob[(long long)o * P + x] = f_to_canonical(-zb, q, qinv, pi.q);
     }
 }
 
