@@ -66,8 +66,9 @@ __device__ __forceinline__ uint64_t inc_prod_slot(const uint64_t* u, const uint6
 }
 
 // d0 = a1 a2, d1 = a1 b2 + b1 a2, d2 = b1 b2 in the NTT domain (mlwe.c:665-709 at rank 1).
-// dd (may be null, split 1 only): also write d0's limb k to dd + b dd_stride + k dd_step
-// -- the spectrum of key-switch digit k modulo its own prime, NTT(INTT(d0_k)) = d0_k.
+// dd (may be null, split 1 only): write d0's limb k to dd + b dd_stride + k dd_step instead
+// of T -- the spectrum of key-switch digit k modulo its own prime, NTT(INTT(d0_k)) = d0_k,
+// from where the inverse transform reads it.
 template <int S>
 __global__ void k_tensor(uint64_t* __restrict__ T, const uint64_t* __restrict__ c1,
                          const uint64_t* __restrict__ c2, const __grid_constant__ LimbPrimes lp,
@@ -107,8 +108,7 @@ __global__ void k_tensor(uint64_t* __restrict__ T, const uint64_t* __restrict__ 
             };
             one(ua1.x, ub1.x, ua2.x, ub2.x, r0.x, r1.x, r2.x);
             one(ua1.y, ub1.y, ua2.y, ub2.y, r0.y, r1.y, r2.y);
-            *reinterpret_cast<ulonglong2*>(t0 + x) = r0;
-            if (d0k) *reinterpret_cast<ulonglong2*>(d0k + x) = r0;
+            *reinterpret_cast<ulonglong2*>((d0k ? d0k : t0) + x) = r0;
             *reinterpret_cast<ulonglong2*>(t0 + x + LN) = r1;
             *reinterpret_cast<ulonglong2*>(t0 + x + 2 * LN) = r2;
         }
@@ -118,8 +118,7 @@ __global__ void k_tensor(uint64_t* __restrict__ T, const uint64_t* __restrict__ 
         for (long long x = blockIdx.x * (long long)blockDim.x + threadIdx.x; x < N;
              x += (long long)gridDim.x * blockDim.x) {
             const uint64_t va1 = a1[x], vb1 = b1[x], va2 = a2[x], vb2 = b2[x];
-            t0[x] = mul_mod(va1, va2, pi);
-            if (d0k) d0k[x] = t0[x];
+            (d0k ? d0k : t0)[x] = mul_mod(va1, va2, pi);
             t0[x + LN] = add_mod(mul_mod(va1, vb2, pi), mul_mod(vb1, va2, pi), pi.q);
             t0[x + 2 * LN] = mul_mod(vb1, vb2, pi);
         }
@@ -476,15 +475,22 @@ __global__ void __launch_bounds__(kColdownThreads, 6) k_coldown(uint64_t* __rest
 // p - N otherwise (gen odd, so N gen = N mod 2N).  Stores are coalesced 16-byte pairs;
 // the scattered 8-byte reads hit the source row in L2.  Index arithmetic is 32-bit
 // (2N <= 2^31, so products wrap correctly modulo 2N).
+constexpr int kGaloisInline = 16;
+struct GaloisIndex {  // gen^-1 by ciphertext: in the launch's parameters for a small batch
+    int in_params;
+    uint64_t ginv[kGaloisInline];
+    const uint64_t* ginvs;
+};
+
 __global__ void k_permute_batch(uint64_t* __restrict__ out, const uint64_t* __restrict__ in,
-                                const uint64_t* __restrict__ ginvs, const __grid_constant__ LimbPrimes lp,
+                                const __grid_constant__ GaloisIndex gi, const __grid_constant__ LimbPrimes lp,
                                 const PrimeInfo* __restrict__ primes, int L, long long N, int log_split) {
     const int by = blockIdx.y;  // (b, c, k)
     const int k = by % L;
     const int bc = by / L;
     const int b = bc >> 1;
     const uint64_t q = primes[lp.p[k]].q;
-    const uint32_t ginv = (uint32_t)ginvs[b];
+    const uint32_t ginv = (uint32_t)(gi.in_params ? gi.ginv[b] : gi.ginvs[b]);
     const uint64_t* src = in + ((long long)bc * L + k) * N;
     uint64_t* dst = out + ((long long)bc * L + k) * N;
     const uint32_t n = (uint32_t)N, mask2n = 2 * n - 1;
@@ -564,10 +570,23 @@ __device__ __forceinline__ void mac2_store(uint64_t* acc, long long b, long long
     *reinterpret_cast<ulonglong2*>(oa + dstride) = rb;
 }
 
-// pairs[k] = b0 | (b1 + 1) << 32 (b1 = -1: b0 alone).
+// The ciphertexts of pair k and their key: pairs (2k, 2k + 1) with one key for all when `one`
+// is set; else pair entries b0 | (b1 + 1) << 32 (b1 = -1: b0 alone) and each ciphertext's key,
+// in the launch's parameters for a small batch and in device memory otherwise.  (A kernel
+// that puts small arrays into device memory first costs 1.4 us of a 45 us multiply.)
+constexpr int kMacInline = 16;
+struct MacIndex {
+    const uint64_t* one;
+    long long batch;
+    int in_params;
+    uint64_t pair[kMacInline];
+    const uint64_t* key[kMacInline];  // by ciphertext
+    const uint64_t* const* keys;      // device arrays
+    const uint64_t* pairs;
+};
+
 __global__ void __launch_bounds__(256) k_mac_paired(uint64_t* __restrict__ acc, const uint64_t* __restrict__ D,
-                                                    const uint64_t* const* __restrict__ keys,
-                                                    const uint64_t* __restrict__ pairs,
+                                                    const __grid_constant__ MacIndex ix,
                                                     const __grid_constant__ LimbPrimes lp,
                                                     const PrimeInfo* __restrict__ primes, int nd, int ne,
                                                     long long N, const __grid_constant__ FoldConsts fold) {
@@ -575,16 +594,25 @@ __global__ void __launch_bounds__(256) k_mac_paired(uint64_t* __restrict__ acc, 
     __shared__ uint64_t bars[kMacStages];
     const int by = blockIdx.y;
     const int bp = by / ne, i = by - bp * ne;
-    const uint64_t pr = pairs[bp];
-    const long long b0 = (long long)(pr & 0xffffffffULL);
-    const long long b1 = (long long)(pr >> 32) - 1;
+    long long b0, b1;
+    const uint64_t* k0;
+    if (ix.one) {
+        b0 = 2LL * bp;
+        b1 = b0 + 1 < ix.batch ? b0 + 1 : -1;
+        k0 = ix.one;
+    } else {
+        const uint64_t pr = ix.in_params ? ix.pair[bp] : ix.pairs[bp];
+        b0 = (long long)(pr & 0xffffffffULL);
+        b1 = (long long)(pr >> 32) - 1;
+        k0 = ix.in_params ? ix.key[b0] : ix.keys[b0];
+    }
     const bool two = b1 >= 0;
     const long long x0 = (long long)blockIdx.x * kMacChunk;
     const long long dstride = (long long)ne * N;
     const long long kstride = (long long)2 * ne * N;
     const uint64_t* d0 = D + b0 * nd * dstride + (long long)i * N + x0;
     const uint64_t* d1 = two ? D + b1 * nd * dstride + (long long)i * N + x0 : nullptr;
-    const uint64_t* ka = keys[b0] + (long long)i * N + x0;
+    const uint64_t* ka = k0 + (long long)i * N + x0;
     if (threadIdx.x == 0) {
         for (int s = 0; s < kMacStages; ++s) mbar_init(&bars[s], 1);
         fence_mbar_init();
@@ -644,13 +672,10 @@ __global__ void __launch_bounds__(256) k_mac_paired(uint64_t* __restrict__ acc, 
 }
 
 // One k_mac launch for the ring's split degree (each split degree is its own kernel,
-// so the pointwise one keeps its small register footprint).
-// keys_aligned: every key polynomial starts on a 16-byte boundary.
-// pairs (device, npairs entries, see k_mac_paired): the staged kernel runs when they are
-// given and its shape conditions hold (mac_staged_ok); k_mac otherwise.
+// so the pointwise one keeps its small register footprint): the shapes k_mac_paired does
+// not take (mac_staged_ok).
 void launch_mac(IncNtt* t, uint64_t* acc, const uint64_t* D, const uint64_t* const* keys, const uint64_t* order,
-                const LimbPrimes& lpe, int nd, int ne, long long N, uint64_t B, cudaStream_t st, bool keys_aligned,
-                const FoldConsts* fold = nullptr, const uint64_t* pairs = nullptr, uint64_t npairs = 0);
+                const LimbPrimes& lpe, int nd, int ne, long long N, uint64_t B, cudaStream_t st);
 
 // Pairs of consecutive ciphertexts (in `order`, or 0..B-1) whose key pointers are
 // equal, singles elsewhere, in k_mac_paired's encoding; returns the count.
@@ -672,8 +697,8 @@ uint64_t key_pairs(const uint64_t* const* keys, const uint64_t* order, uint64_t 
     return n;
 }
 
-// Whether launch_mac, given key pairs, takes the staged pointwise kernel (the only one
-// that folds pass-through components): split 1, FP64 primes, aligned rows, N a multiple
+// Whether the staged pointwise kernel (the only one that folds pass-through components)
+// takes a multiply-accumulate: split 1, FP64 primes, aligned rows, N a multiple
 // of the chunk.
 bool mac_staged_ok(IncNtt* t, const uint64_t* acc, const uint64_t* D, const LimbPrimes& lpe, int ne, long long N,
                    bool keys_aligned);
@@ -696,19 +721,17 @@ bool mac_staged_ok(IncNtt* t, const uint64_t* acc, const uint64_t* D, const Limb
     return pointwise && N % kMacChunk == 0 && prepare_ckks_kernels() == 0;
 }
 
+void launch_mac_staged(IncNtt* t, uint64_t* acc, const uint64_t* D, const MacIndex& ix, uint64_t npairs,
+                       const LimbPrimes& lpe, int nd, int ne, long long N, cudaStream_t st, const FoldConsts* fold) {
+    note_launch();
+    FoldConsts none;
+    memset(&none, 0, sizeof none);
+    const dim3 g((unsigned)(N / kMacChunk), (unsigned)(npairs * ne), 1);
+    k_mac_paired<<<g, kMacChunk / 2, kMacSmem, st>>>(acc, D, ix, lpe, t->d_info, nd, ne, N, fold ? *fold : none);
+}
+
 void launch_mac(IncNtt* t, uint64_t* acc, const uint64_t* D, const uint64_t* const* keys, const uint64_t* order,
-                const LimbPrimes& lpe, int nd, int ne, long long N, uint64_t B, cudaStream_t st, bool keys_aligned,
-                const FoldConsts* fold, const uint64_t* pairs, uint64_t npairs) {
-    // (the callers that fold pass-through components check mac_staged_ok and pass pairs)
-    if (pairs && npairs && mac_staged_ok(t, acc, D, lpe, ne, N, keys_aligned)) {
-        note_launch();
-        FoldConsts none;
-        memset(&none, 0, sizeof none);
-        const dim3 g((unsigned)(N / kMacChunk), (unsigned)(npairs * ne), 1);
-        k_mac_paired<<<g, kMacChunk / 2, kMacSmem, st>>>(acc, D, keys, pairs, lpe, t->d_info, nd, ne, N,
-                                                          fold ? *fold : none);
-        return;
-    }
+                const LimbPrimes& lpe, int nd, int ne, long long N, uint64_t B, cudaStream_t st) {
     const dim3 g = grid_xy(N, (long long)B * ne);
     switch (t->pub.split_degree) {
         case 1: k_mac<1><<<g, 256, 0, st>>>(acc, D, keys, order, lpe, t->d_info, nd, ne, N); break;
@@ -813,27 +836,6 @@ int blocks_transform(IncNtt* t, uint64_t* data, uint64_t count, const uint32_t* 
     rs.batch = (int)count;
     rs.batch_stride = (long long)nl * N;
     rs.in_batch_stride = rs.batch_stride;
-    mark_fp64(rs, t);
-    return launch_ntt(rs, t->d_info, inverse, st);
-}
-
-// In-place transform of the first [nl][N] block of `count` polynomials `stride` apart.
-int strided_transform(IncNtt* t, uint64_t* data, uint64_t count, long long stride, const uint32_t* lim, int nl,
-                      bool inverse, cudaStream_t st) {
-    const long long N = (long long)t->pub.N;
-    RowSet rs;
-    memset(&rs, 0, sizeof rs);
-    for (int i = 0; i < nl; ++i) {
-        rs.in[i] = data + (long long)i * N;
-        rs.out[i] = data + (long long)i * N;
-        rs.prime[i] = lim[i];
-    }
-    rs.nlimbs = nl;
-    rs.split = (int)t->pub.split_degree;
-    rs.logP = t->logP;
-    rs.batch = (int)count;
-    rs.batch_stride = stride;
-    rs.in_batch_stride = stride;
     mark_fp64(rs, t);
     return launch_ntt(rs, t->d_info, inverse, st);
 }
@@ -1212,9 +1214,7 @@ int mac_one_sample(IncNtt* t, uint64_t* acc, const uint64_t* D, const uint64_t* 
     const uint64_t kp = (uint64_t)(uintptr_t)keys;
     const int e = upload_small(keyptr, &kp, 1, st);
     if (e) return e;
-    const bool aligned = (reinterpret_cast<uintptr_t>(keys) & 15) == 0;
-    launch_mac(t, acc, D, (const uint64_t* const*)keyptr, nullptr, lpe, nd, ne, (long long)t->pub.N, 1, st, aligned,
-               nullptr, nullptr, 0);
+    launch_mac(t, acc, D, (const uint64_t* const*)keyptr, nullptr, lpe, nd, ne, (long long)t->pub.N, 1, st);
     return (int)cudaGetLastError();
 }
 
@@ -1243,9 +1243,6 @@ int ckks_mul_relin_rescale(IncNtt* t, uint64_t* out, const uint64_t* ct1, const 
     uint64_t* acc = D + B * (uint64_t)nl * ne * N;      // [B][2][ne][N]
     uint64_t* keyptrs = acc + B * 2 * ne * N;           // [B]
 
-    uint64_t* d_pairs = keyptrs + B;                    // [B]
-    std::vector<const uint64_t*> kp(B, rlk);
-    if (!check_cuda(upload_small(keyptrs, (const uint64_t*)kp.data(), B, st), where)) return 1;
     const bool rlk_aligned = (reinterpret_cast<uintptr_t>(rlk) & 15) == 0;
     // When the staged MAC runs: d1 and d2 pass through the key switch and stay in the
     // NTT domain, folded into the accumulator (FoldConsts), so only d0 -- whose limbs are
@@ -1268,7 +1265,22 @@ int ckks_mul_relin_rescale(IncNtt* t, uint64_t* out, const uint64_t* ct1, const 
     }
     if (!check_cuda(cudaGetLastError(), where)) return 1;
     if (fold) {
-        if (!check_cuda(strided_transform(t, T, B, 3LL * nl * N, limbs, nl, true, st), where)) return 1;
+        // d0 back to coefficients: from the digit buffer's own-prime rows into T
+        RowSet rs;
+        memset(&rs, 0, sizeof rs);
+        for (int i = 0; i < nl; ++i) {
+            rs.in[i] = D + (long long)i * (ne + 1) * N;
+            rs.out[i] = T + (long long)i * N;
+            rs.prime[i] = limbs[i];
+        }
+        rs.nlimbs = nl;
+        rs.split = 1;
+        rs.logP = t->logP;
+        rs.batch = (int)B;
+        rs.in_batch_stride = (long long)nl * ne * N;
+        rs.batch_stride = 3LL * nl * N;
+        mark_fp64(rs, t);
+        if (!check_cuda(launch_ntt(rs, t->d_info, true, st), where)) return 1;
     } else {
         if (!check_cuda(blocks_transform(t, T, 3 * B, limbs, nl, true, st), where)) return 1;
     }
@@ -1288,12 +1300,17 @@ int ckks_mul_relin_rescale(IncNtt* t, uint64_t* out, const uint64_t* ct1, const 
             fc.pfq[i] = fc.pf[i] / (double)q;
         }
     }
-    // every ciphertext uses the relinearisation key: pairs (0, 1), (2, 3), ...
-    std::vector<uint64_t> pairs(B);
-    const uint64_t npairs = key_pairs(kp.data(), nullptr, B, pairs.data());
-    if (!check_cuda(upload_small(d_pairs, pairs.data(), npairs, st), where)) return 1;
-    launch_mac(t, acc, D, (const uint64_t* const*)keyptrs, nullptr, lpe, nl, ne, N, B, st, rlk_aligned,
-               fold ? &fc : nullptr, d_pairs, npairs);
+    if (fold) {
+        MacIndex ix;
+        memset(&ix, 0, sizeof ix);
+        ix.one = rlk;
+        ix.batch = (long long)B;
+        launch_mac_staged(t, acc, D, ix, (B + 1) / 2, lpe, nl, ne, N, st, &fc);
+    } else {
+        std::vector<const uint64_t*> kp(B, rlk);
+        if (!check_cuda(upload_small(keyptrs, (const uint64_t*)kp.data(), B, st), where)) return 1;
+        launch_mac(t, acc, D, (const uint64_t* const*)keyptrs, nullptr, lpe, nl, ne, N, B, st);
+    }
     if (!check_cuda(cudaGetLastError(), where)) return 1;
     const ModDownConsts mc = moddown_consts(t, limbs, nl, special);
     const int use_pass = fold ? 0 : 1;
@@ -1340,7 +1357,11 @@ int ckks_rotate(IncNtt* t, uint64_t* out, const uint64_t* ct, uint64_t B, const 
     uint64_t* d_gens = keyptrs + B;                     // [B]
     uint64_t* d_order = d_gens + B;                     // [B]
     uint64_t* d_pairs = d_order + B;                    // [B]
-    if (!check_cuda(upload_small(keyptrs, (const uint64_t*)gks, B, st), where)) return 1;
+    bool keys_aligned = true;
+    for (uint64_t b = 0; b < B; ++b) keys_aligned = keys_aligned && (reinterpret_cast<uintptr_t>(gks[b]) & 15) == 0;
+    const bool staged = mac_staged_ok(t, acc, D, lpe, ne, N, keys_aligned);
+    const bool small = B <= (uint64_t)kMacInline;
+    if (!(staged && small) && !check_cuda(upload_small(keyptrs, (const uint64_t*)gks, B, st), where)) return 1;
     // ciphertexts grouped by key (stable), so each key is read from HBM about once
     std::vector<uint64_t> order(B);
     for (uint64_t b = 0; b < B; ++b) order[b] = b;
@@ -1349,7 +1370,7 @@ int ckks_rotate(IncNtt* t, uint64_t* out, const uint64_t* ct, uint64_t B, const 
     });
     bool identity = true;
     for (uint64_t b = 0; b < B && identity; ++b) identity = order[b] == b;
-    if (!identity && !check_cuda(upload_small(d_order, order.data(), B, st), where)) return 1;
+    if (!staged && !identity && !check_cuda(upload_small(d_order, order.data(), B, st), where)) return 1;
     const uint64_t* src = ct;
     if (gens) {
         // the gather needs gen^-1 mod 2N (Newton's iteration doubles the correct low bits)
@@ -1359,21 +1380,40 @@ int ckks_rotate(IncNtt* t, uint64_t* out, const uint64_t* ct, uint64_t B, const 
             for (int it = 0; it < 6; ++it) x *= 2 - gens[b] * x;
             ginv[b] = x & (2 * (uint64_t)N - 1);
         }
-        if (!check_cuda(upload_small(d_gens, ginv.data(), B, st), where)) return 1;
-        k_permute_batch<<<grid_xy((N + 1) / 2, (long long)B * 2 * nl), 256, 0, st>>>(Pm, ct, d_gens, lp, t->d_info, nl,
-                                                                                N, ls);
+        GaloisIndex gi;
+        memset(&gi, 0, sizeof gi);
+        if (small) {
+            gi.in_params = 1;
+            for (uint64_t b = 0; b < B; ++b) gi.ginv[b] = ginv[b];
+        } else {
+            gi.ginvs = d_gens;
+            if (!check_cuda(upload_small(d_gens, ginv.data(), B, st), where)) return 1;
+        }
+        k_permute_batch<<<grid_xy((N + 1) / 2, (long long)B * 2 * nl), 256, 0, st>>>(Pm, ct, gi, lp, t->d_info, nl, N, ls);
         if (!check_cuda(cudaGetLastError(), where)) return 1;
         src = Pm;
     }
     if (!check_cuda(digits_forward(t, D, src, 2LL * nl * N, B, ext, nl, ne, st), where)) return 1;
-    bool keys_aligned = true;
-    for (uint64_t b = 0; b < B; ++b) keys_aligned = keys_aligned && (reinterpret_cast<uintptr_t>(gks[b]) & 15) == 0;
-    // ciphertexts that share a Galois key (adjacent in the key-grouped order) in pairs
-    std::vector<uint64_t> pairs(B);
-    const uint64_t npairs = key_pairs(gks, order.data(), B, pairs.data());
-    if (!check_cuda(upload_small(d_pairs, pairs.data(), npairs, st), where)) return 1;
-    launch_mac(t, acc, D, (const uint64_t* const*)keyptrs, identity ? nullptr : d_order, lpe, nl, ne, N, B, st,
-               keys_aligned, nullptr, d_pairs, npairs);
+    if (staged) {
+        // ciphertexts that share a Galois key (adjacent in the key-grouped order) in pairs
+        std::vector<uint64_t> pairs(B);
+        const uint64_t npairs = key_pairs(gks, order.data(), B, pairs.data());
+        MacIndex ix;
+        memset(&ix, 0, sizeof ix);
+        ix.batch = (long long)B;
+        if (small) {
+            ix.in_params = 1;
+            for (uint64_t k = 0; k < npairs; ++k) ix.pair[k] = pairs[k];
+            for (uint64_t b = 0; b < B; ++b) ix.key[b] = gks[b];
+        } else {
+            ix.keys = (const uint64_t* const*)keyptrs;
+            ix.pairs = d_pairs;
+            if (!check_cuda(upload_small(d_pairs, pairs.data(), npairs, st), where)) return 1;
+        }
+        launch_mac_staged(t, acc, D, ix, npairs, lpe, nl, ne, N, st, nullptr);
+    } else {
+        launch_mac(t, acc, D, (const uint64_t* const*)keyptrs, identity ? nullptr : d_order, lpe, nl, ne, N, B, st);
+    }
     if (!check_cuda(cudaGetLastError(), where)) return 1;
     const ModDownConsts mc = moddown_consts(t, limbs, nl, special);
     return check_cuda(acc_inverse_moddown(t, out, acc, B, ext, ne, mc, src, 2LL * nl * N, 0, (long long)nl * N, 0, 1, 0, st),
