@@ -132,3 +132,22 @@ def test_chain_falls_back_for_other_shapes(cuda):
     torch.cuda.synchronize()
     assert np.array_equal(out.cpu().numpy().view(np.uint64),
                           _separate_launches(cuda, small, ua.contiguous(), ub.contiguous()))
+
+
+@pytest.mark.parametrize("N,split,sizes,B", [
+    (2048, 4, [50], 1), (2048, 4, [50, 50, 50], 100), (4096, 4, [50], 147), (4096, 4, [50], 148), (4096, 4, [50], 149),
+    (4096, 2, [50], 149), (4096, 8, [50, 45], 74), (4096, 8, [50], 149),
+])
+def test_chain_threads_of_8_residues(cuda, N, split, sizes, B):
+    """Shapes on both sides of the row counts where a row gets twice the threads."""
+    from vfhe_b200.arith import Ring
+    from vfhe_b200.batch import to_device
+
+    ring = Ring(N, prime_size=sizes, split_degree=split, engine=cuda)
+    rng = np.random.default_rng(N + 10 * split + B)
+    ta = to_device(_rows(ring, B, rng, extremes=True))
+    tb = to_device(_rows(ring, B, rng, extremes=True))
+    got, launches = _chain(cuda, ring, ta, tb)
+    assert launches == 1
+    assert np.array_equal(got, _separate_launches(cuda, ring, ta, tb)), (N, split, B)
+    cuda.check("chain of 8 residues a thread")

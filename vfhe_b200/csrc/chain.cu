@@ -22,7 +22,7 @@
 #include <mutex>
 
 #include "engine.cuh"
-#include "ntt_f64_dev.cuh"
+#include "ntt_f64_r8.cuh"
 
 namespace vc {
 
@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(S << (K - 4), (S << (K - 4)) <= 256 ? 2 : 1) k
     constexpr int TPT = 1 << (K - 4), P = 1 << K, PADDED = P + (P >> 4);
     constexpr bool GROUP = S > 1;
     extern __shared__ __align__(128) double csm[];
-    double* spec = csm;            // [S][PADDED]: a's spectra, reduced, at pad(edge<K>(t, m))
+    double* spec = csm;            // [S][PADDED]: a's spectra, reduced, at pad(edge_base) + pad(edge_step)
     double* ex = csm + S * PADDED;  // [S][PADDED]: each block's exchanges, then b's spectra
     const int g = threadIdx.x / TPT;
     const int t = threadIdx.x - g * TPT;
@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(S << (K - 4), (S << (K - 4)) <= 256 ? 2 : 1) k
     const double q = pi.qd, qinv = pi.qinv;
     const long long off = row * (long long)(S * P) + (long long)g * P;
     double* exg = ex + g * PADDED;
+    const int eb = edge_base<K>(t), pe = pad(eb);  // steps have bits that bases lack: pad adds up
 
     Tile tile;
     tile.hi = 0;
@@ -63,7 +64,7 @@ __global__ void __launch_bounds__(S << (K - 4), (S << (K - 4)) <= 256 ? 2 : 1) k
     tile.src = a + off;
     tile_fwd_regs<K, false, false, GROUP>(tile, K, false, exg, t, x, g);
 #pragma unroll
-    for (int m = 0; m < 16; ++m) spec[g * PADDED + pad(edge<K>(t, m))] = f_reduce(x[m], q, qinv);
+    for (int m = 0; m < 16; ++m) spec[g * PADDED + pe + pad(edge_step<K>(m))] = f_reduce(x[m], q, qinv);
     tile_sync<K, GROUP>(g);  // the block's last exchange reads are over before b's first write
     // b's block g.  Its twiddles are a's again; the prime's address goes through an
     // opaque move so that the compiler reloads them instead of keeping a's ~90 registers
@@ -78,17 +79,17 @@ __global__ void __launch_bounds__(S << (K - 4), (S << (K - 4)) <= 256 ? 2 : 1) k
 #pragma unroll
         for (int m = 0; m < 16; ++m) {
             const double w = f_reduce(x[m], q, qinv);
-            x[m] = f_mulmod(spec[pad(edge<K>(t, m))], w, __dmul_rn(w, qinv), q);  // |x| <= 3q/4
+            x[m] = f_mulmod(spec[pe + pad(edge_step<K>(m))], w, __dmul_rn(w, qinv), q);  // |x| <= 3q/4
         }
     } else {
         tile_sync<K, GROUP>(g);  // the block's exchanges are over: its buffer takes b's spectrum
 #pragma unroll
-        for (int m = 0; m < 16; ++m) exg[pad(edge<K>(t, m))] = f_reduce(x[m], q, qinv);
+        for (int m = 0; m < 16; ++m) exg[pe + pad(edge_step<K>(m))] = f_reduce(x[m], q, qinv);
         __syncthreads();  // every block's spectra of a and b are in shared memory
-        const ulonglong2* tw = reinterpret_cast<const ulonglong2*>(pi.twist);
+        const ulonglong2* tw = reinterpret_cast<const ulonglong2*>(pi.twist) + eb;
 #pragma unroll
         for (int m = 0; m < 16; ++m) {
-            const int xs = edge<K>(t, m), px = pad(xs);
+            const int px = pe + pad(edge_step<K>(m));
             double acc = 0.0, wrap = 0.0;
 #pragma unroll
             for (int i = 0; i < S; ++i) {
@@ -104,7 +105,7 @@ __global__ void __launch_bounds__(S << (K - 4), (S << (K - 4)) <= 256 ? 2 : 1) k
             // at most 8 terms of at most 3q/4 each: below 6q < 2^53
             acc = f_reduce(acc, q, qinv);
             wrap = f_reduce(wrap, q, qinv);
-            const uint64_t wi = tw[xs].x;
+            const uint64_t wi = tw[edge_step<K>(m)].x;
             const double wd = wi > pi.q / 2 ? (double)wi - q : (double)wi;
             x[m] = f_reduce(__dadd_rn(acc, f_mulmod(wrap, wd, __dmul_rn(wd, qinv), q)), q, qinv);
         }
@@ -116,16 +117,108 @@ __global__ void __launch_bounds__(S << (K - 4), (S << (K - 4)) <= 256 ? 2 : 1) k
     for (int m = 0; m < 16; ++m) o[own<K - 4>(t, m)] = f_to_canonical(x[m], q, qinv, pi.q);
 }
 
+// The same chain with 8 residues a thread (ntt_f64_r8.cuh): twice the warps a row, for the
+// shapes whose rows leave an SM too few of them (16 residues: 4 warps a row at (K, S) = (9, 4),
+// 8 at (10, 4)).  The kernel is bound by one block's chain of exchanges and barriers there,
+// not by FP64 issue.  Three limbs, 16 -> 8 residues a thread, us per call with its launch:
+//   (9, 4)   48 rows 13.4 -> 10.5, 192 rows 16.5 -> 14.4, 1200 rows 61.7 -> 50.5
+//   (10, 4)  48 rows 16.5 -> 14.4, 144 rows 16.6 -> 14.4, 192 rows 24.7 -> 24.7, 1200 rows 96 -> 104
+//   (11, 2)  48 rows 16.5 -> 14.5, 144 rows 16.5 -> 15.5, 1200 rows 104 -> 116
+//   (12, 1)  48 rows 12.4 -> 14.4; (11, 1) and (10, 2) equal; 1024 threads spill (1.5x slower)
+// Hence chain8_rows.
+template <int K, int S>
+__global__ void __launch_bounds__(S << (K - 3), S << (K - 3) <= 256 ? 2 : 1)
+    k_chain8_f(uint64_t* __restrict__ out, const uint64_t* __restrict__ a, const uint64_t* __restrict__ b,
+               const __grid_constant__ ChainLimbs cl, const PrimeInfo* __restrict__ primes, int nl) {
+    constexpr int TPT = 1 << (K - 3), P = 1 << K, PADDED = P + (P >> 3), NP = Passes8<K>::count;
+    extern __shared__ __align__(128) double csm[];
+    double* spec = csm;             // [S][PADDED]: a's spectra, reduced
+    double* ex = csm + S * PADDED;  // [S][PADDED]: each block's exchanges, then b's spectra
+    const int g = threadIdx.x / TPT, t = threadIdx.x - g * TPT;
+    const long long row = blockIdx.x;  // polynomial * nl + limb slot
+    const PrimeInfo& pi = primes[cl.p[(int)(row % nl)]];
+    const double q = pi.qd, qinv = pi.qinv;
+    const double2* fwd = reinterpret_cast<const double2*>(pi.fwd_d);
+    const long long off = row * (long long)(S * P) + (long long)g * P;
+    double* exg = ex + g * PADDED;
+    double* specg = spec + g * PADDED;
+    double x[8];
+    Twiddles8 tw;
+    load_twiddles<K, 0>(tw, fwd, t);
+#pragma unroll
+    for (int m = 0; m < 8; ++m) x[m] = f_from_u64(a[off + Pass8<K, 0>::index(t, m)]);
+    fwd8<K, 0>(x, tw, exg, t, g, fwd, q, qinv);
+#pragma unroll
+    for (int m = 0; m < 8; ++m) specg[pad8(Pass8<K, NP - 1>::index(t, m))] = f_reduce(x[m], q, qinv);
+#pragma unroll
+    for (int m = 0; m < 8; ++m) x[m] = f_from_u64(b[off + Pass8<K, 0>::index(t, m)]);
+    load_twiddles<K, 0>(tw, fwd, t);
+    fwd8<K, 0>(x, tw, exg, t, g, fwd, q, qinv);
+    group_sync(g, TPT);  // the block's exchanges are over: its buffer takes b's spectrum
+#pragma unroll
+    for (int m = 0; m < 8; ++m) exg[pad8(Pass8<K, NP - 1>::index(t, m))] = f_reduce(x[m], q, qinv);
+    __syncthreads();  // every block's spectra of a and b are in shared memory
+    const ulonglong2* twist = reinterpret_cast<const ulonglong2*>(pi.twist);
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+        const int xs = Pass8<K, NP - 1>::index(t, m), px = pad8(xs);
+        double acc = 0.0, wrap = 0.0;
+#pragma unroll
+        for (int i = 0; i < S; ++i) {
+            const double u = spec[i * PADDED + px];
+            const int k = i <= g ? g - i : g - i + S;
+            const double v = ex[k * PADDED + px];
+            const double p = f_mulmod(u, v, __dmul_rn(v, qinv), q);
+            if (i <= g) acc = __dadd_rn(acc, p);
+            else wrap = __dadd_rn(wrap, p);
+        }
+        // at most 8 terms of at most 3q/4 each: below 6q < 2^53
+        acc = f_reduce(acc, q, qinv);
+        wrap = f_reduce(wrap, q, qinv);
+        const uint64_t wi = twist[xs].x;
+        const double wd = wi > pi.q / 2 ? (double)wi - q : (double)wi;
+        x[m] = f_reduce(__dadd_rn(acc, f_mulmod(wrap, wd, __dmul_rn(wd, qinv), q)), q, qinv);
+    }
+    __syncthreads();  // every block's b spectrum is read before the exchanges reuse it
+    Twiddles8 twi;
+    load_twiddles<K, NP - 1>(twi, reinterpret_cast<const double2*>(pi.inv_d), t);
+    inv8<K, NP - 1>(x, twi, exg, t, g, pi);
+#pragma unroll
+    for (int m = 0; m < 8; ++m) out[off + Pass8<K, 0>::index(t, m)] = f_to_canonical(x[m], q, qinv, pi.q);
+}
+
+template <int K, int S>
+constexpr size_t chain8_smem() {
+    return sizeof(double) * 2 * (size_t)S * ((1 << K) + (1 << (K - 3)));
+}
+
 template <int K, int S>
 constexpr size_t chain_smem() {
     return sizeof(double) * 2 * (size_t)S * ((1 << K) + (1 << (K - 4)));
 }
 
+// Most rows the 8-residue kernel takes: any number at (9, 4), one row an SM where a row is
+// 512 threads in split blocks (two of the 16-residue kernel's CTAs share an SM beyond that),
+// none elsewhere.
+template <int K, int S>
+long long chain8_rows() {
+    if constexpr (K == 9 && S == 4) return 0x7fffffffLL;
+    else if constexpr (S > 1 && S << (K - 3) == 512) return sm_count();
+    else return 0;
+}
+
 template <int K, int S>
 int chain_attr() {
-    if (chain_smem<K, S>() <= 48 * 1024) return 0;
-    return (int)cudaFuncSetAttribute(k_chain_f<K, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)chain_smem<K, S>());
+    int e = 0;
+    if (chain_smem<K, S>() > 48 * 1024)
+        e = (int)cudaFuncSetAttribute(k_chain_f<K, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)chain_smem<K, S>());
+    if constexpr (S > 1 && S << (K - 3) <= 512) {
+        if (!e && chain8_smem<K, S>() > 48 * 1024)
+            e = (int)cudaFuncSetAttribute(k_chain8_f<K, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)chain8_smem<K, S>());
+    }
+    return e;
 }
 
 template <int K, int S>
@@ -137,7 +230,12 @@ int chain_launch(uint64_t* out, const uint64_t* a, const uint64_t* b, long long 
     static int attr_err = 0;
     std::call_once(once, [] { attr_err = chain_attr<K, S>(); });
     if (attr_err) return attr_err;
-    k_chain_f<K, S><<<(unsigned)rows, S << (K - 4), chain_smem<K, S>(), st>>>(out, a, b, cl, d, nl);
+    bool eight = false;
+    if constexpr (S > 1 && S << (K - 3) <= 512) {
+        eight = rows <= chain8_rows<K, S>();
+        if (eight) k_chain8_f<K, S><<<(unsigned)rows, S << (K - 3), chain8_smem<K, S>(), st>>>(out, a, b, cl, d, nl);
+    }
+    if (!eight) k_chain_f<K, S><<<(unsigned)rows, S << (K - 4), chain_smem<K, S>(), st>>>(out, a, b, cl, d, nl);
     note_launch();
     return (int)cudaGetLastError();
 }
