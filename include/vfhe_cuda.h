@@ -444,7 +444,8 @@ int vfhe_cuda_prng_blocks(uint32_t *d_out, uint64_t nblocks, const uint32_t *key
  *   d_tv    [2][L0][N]       LUT test vector (rank-1 MLWE), coefficient domain
  *   d_out_a [batch][L0][N]   extracted masks; d_out_b [batch][L0] extracted bodies.
  * torus_base is the LUT size t (rot_b uses floor(Q / 4t), cggi16.py:65).  The n
- * rotation steps run as one CUDA graph, captured at the first call per shape. */
+ * rotation steps run in one launch (a cluster per ciphertext) for small batches, else as
+ * one CUDA graph, captured at the first call per shape. */
 uint64_t vfhe_cuda_cggi_workspace_bytes(void *ntt, uint64_t batch, uint32_t n, uint32_t nlimbs);
 int vfhe_cuda_cggi_bootstrap_batch(void *ntt, uint64_t *d_out_a, uint64_t *d_out_b, const uint64_t *d_in_a,
                                    const uint64_t *d_in_b, uint64_t batch, uint32_t n, const uint32_t *limbs,
@@ -540,7 +541,7 @@ int vfhe_cuda_worklist_phase_ms(void *wl, double *out6);
  *   extracted LWEs; d_bsk_f [n][2 levels][2][N/2] spectra of GGSW(s_i), row (c, l) at
  *   c * levels + l; d_tv [N] test vector; rotation offset 2^32 / (4 torus_base).
  *   One persistent launch: every CTA runs whole blind rotations with its accumulator
- *   in shared memory.
+ *   in shared memory (wider CTAs for at most one ciphertext per SM).
  * keyswitch_batch: d_in [batch][N+1] -> d_out [batch][n+1] with d_ksk [N][levels][n+1]
  *   (base 2^base_log, signed digits); exact integer arithmetic.
  * external_product: d_out[b] = ExtProd(GGSW spectra d_ggsw_f, GLWE d_c[b] [2][N]) rounded

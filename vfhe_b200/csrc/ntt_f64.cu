@@ -8,7 +8,8 @@
 //
 // Range schedule (every modular product needs its input below 2^52 in magnitude):
 //   forward (CT: x +- w y): each stage adds at most 3q/4, so passes of <= 4 stages
-//     starting from |x| <= q stay below 4q; all residues are reduced at pass end;
+//     starting from |x| <= q stay below 4q; residues are reduced at pass end, except before a
+//     last pass of at most two stages (f_fwd_bits) and for primes below 2^47;
 //   inverse (GS: x + y, w (x - y)): sums double, so the sum outputs are reduced after
 //     every second stage and at pass end; products are always <= 3q/4.
 #include <cooperative_groups.h>
