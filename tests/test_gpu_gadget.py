@@ -69,3 +69,38 @@ def test_limbs_with_gaps_match_the_oracle(cuda, oracle_engine, N, split, rank):
             outs.append([np.stack([m.component_rows(c) for c in range(rank + 1)]) for m in (sw, prod)])
     for got, want in zip(*outs):
         assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("split", [1, 2])
+def test_digit_of_a_large_prime_outside_the_key(cuda, oracle_engine, split):
+    """A ciphertext limb of a 58-bit prime, whose digit is no double, under a key without that
+    limb: the external product still equals the oracle's."""
+    from vfhe_b200.arith import Ring, repr as domain
+    from vfhe_b200.mlwe import MLWE, MLWE_Scheme
+    from vfhe_b200.native import use_engine
+
+    N, outs = 2**9, []
+    for eng in (cuda, oracle_engine):
+        with use_engine(eng):
+            rng = np.random.default_rng(split)
+            q = Ring(N, prime_size=[50, 45, 58, 40], split_degree=split).primes
+            lims, key_lims = [q[0], q[2], q[3]], [q[0], q[1], q[3]]
+
+            def ring(primes):
+                return Ring(N, prime_size=[int(p).bit_length() for p in primes], primes=primes, split_degree=split)
+
+            s = MLWE_Scheme([ring(lims)], special_rings=[ring(key_lims)], module_rank=1)
+
+            def sample(r):
+                m = MLWE(s, ring=r)
+                for c in range(2):
+                    m.set_component_rows(c, np.stack([rng.integers(0, p, N, dtype=np.uint64) for p in r.primes]))
+                return m
+
+            rows = [sample(s.special_rings[0]) for _ in range(6)]
+            ct, out = sample(s.rings[0]), MLWE(s, ring=s.special_rings[0])
+            ct.repr = domain.coeff
+            eng.lib.mgsw_external_product(out.obj, eng.ffi.new("void*[]", [r.obj for r in rows]), ct.obj, 3, 0)
+            eng.check("mgsw_external_product")
+            outs.append(np.stack([out.component_rows(c) for c in range(2)]))
+    assert np.array_equal(*outs)

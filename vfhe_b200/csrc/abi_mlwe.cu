@@ -256,8 +256,9 @@ int launch_gadget_mac(const GadgetMac& gm, const uint64_t* D, const PrimeInfo* p
     return (int)cudaGetLastError();
 }
 
-// Whether gadget_mac_all takes these operands: one pool, FP64 primes, every key polynomial
-// active at the same extended limbs, blocks apart from one another and the digits.
+// Whether gadget_mac_all takes these operands: one pool, FP64 primes (the digits' own too: a
+// digit is read as a double before it is reduced), every key polynomial active at the same
+// extended limbs, blocks apart from one another and the digits.
 bool gadget_all_ok(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly) {
     IncNtt* t = pool(out);
     const uint64_t ext = ksk[0]->b->rns_mask, mask = poly->pub.rns_mask;
@@ -271,6 +272,9 @@ bool gadget_all_ok(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly) {
     const int ne = mask_indices(ext, t->pub.l, idx);
     for (int i = 0; i < ne; ++i)
         if (!t->info[idx[i]].fp64) return false;
+    uint32_t dig[64];
+    for (int j = 0, n = mask_indices(mask, t->pub.l, dig); j < n; ++j)
+        if (!t->info[dig[j]].fp64) return false;
     if (ne == 0 || t->logP < 8 || t->logP > 17) return false;
     for (int c = 0; c < comps; ++c) {
         Poly* o = P_(c < (int)out->r ? out->a[c] : out->b);
