@@ -192,3 +192,26 @@ def test_keyswitch_tiles_and_shares(cuda, torus_oracle, n, N, base_log, levels, 
         u32(out), u32(d_in), batch, u32(d_k), N, n, base_log, levels,
         cuda.ffi.cast("void*", torch.cuda.current_stream().cuda_stream)) == 0
     assert np.array_equal(to_host(out), oracle_keyswitch(torus_oracle, ext, ksk, p))
+
+
+@pytest.mark.parametrize("base_log,levels", [(8, 2), (9, 1), (9, 3), (10, 2), (15, 2), (16, 1), (16, 2), (23, 1),
+                                             (24, 1), (32, 1)])
+@pytest.mark.parametrize("n,N,batch", [(37, 33, 1), (64, 96, 33), (40, 70, 150)])
+def test_keyswitch_digits_wider_than_a_byte(cuda, torus_oracle, n, N, batch, base_log, levels):
+    """Digits past 8 bits, at the sizes where they take another byte; extreme masks among them."""
+    import torch
+
+    from vfhe_b200.cggi_fft import TorusParams, to_device, to_host
+
+    p = TorusParams(n=n, N=N, ks_base_log=base_log, ks_levels=levels)
+    rng = np.random.default_rng(n + base_log)
+    ksk = rng.integers(0, 1 << 32, (N, levels, n + 1), dtype=np.uint64).astype(np.uint32)
+    ext = rng.integers(0, 1 << 32, (batch, N + 1), dtype=np.uint64).astype(np.uint32)
+    ext[0, :4] = (0x7FFFFFFF, 0x80000000, 0x80000001, 0xFFFFFFFF)
+    d_in, d_k = to_device(ext), to_device(ksk)
+    out = torch.full((batch, n + 1), -1, dtype=torch.int32, device="cuda")
+    u32 = lambda t: cuda.ffi.cast("uint32_t*", t.data_ptr())  # noqa: E731
+    assert cuda.lib.vfhe_cuda_cggi_fft_keyswitch_batch(
+        u32(out), u32(d_in), batch, u32(d_k), N, n, base_log, levels,
+        cuda.ffi.cast("void*", torch.cuda.current_stream().cuda_stream)) == 0
+    assert np.array_equal(to_host(out), oracle_keyswitch(torus_oracle, ext, ksk, p))

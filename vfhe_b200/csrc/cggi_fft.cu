@@ -710,6 +710,9 @@ __global__ void __launch_bounds__((1 << LOGM) / 8) k_rows_to_fourier(double2* __
 // bodies; the launcher splits the mask where ciphertexts x columns leave SMs idle.
 // Measured at n = 630, N = 1024, 8 levels, against 32-bit multiply-adds on 32 ciphertexts
 // x 128 columns a block over the whole mask: 7 ciphertexts 3100 -> 26 us, 4096 3400 -> 984.
+// Digits of more than 8 bits (PARTS > 1) are taken apart into balanced bytes, byte i meeting
+// the key word 2^(8 i): d + sum 128 2^(8 i) has the bytes plus 128, which PARTS bytes hold for
+// d in [-2^(b-1), 2^(b-1)) when b <= 8 PARTS - 1; with four bytes it holds modulo 2^32 for any b.
 constexpr int KS_J = 32;       // mask coefficients decomposed per round
 constexpr int KS_COLS = 32;    // columns per block
 
@@ -741,13 +744,14 @@ __device__ __forceinline__ void byte_planes(uint32_t (&b)[4], uint32_t w0, uint3
 }
 
 // MT: 16-row tiles of ciphertexts a warp takes; the block takes MROWS = 16 MT x 2.
-template <int MT>
+template <int MT, int PARTS>
 __global__ void __launch_bounds__(256) k_cggi_keyswitch(uint32_t* __restrict__ out, const uint32_t* __restrict__ in,
                                                         long long B, const uint32_t* __restrict__ ksk, int Nin, int n,
                                                         int base_log, int levels, int j_share) {
     constexpr int MROWS = 32 * MT;
     extern __shared__ __align__(16) unsigned char ksm[];
-    const int kc = KS_J * levels;  // digits of one round, a multiple of 32
+    const int dj = levels * PARTS;  // digit bytes of one mask coefficient
+    const int kc = KS_J * dj;       // of one round, a multiple of 32
     const int pitch = kc + 16;     // bytes; the 16 keep a fragment's 8 rows on different banks
     int8_t* dig = reinterpret_cast<int8_t*>(ksm);  // [MROWS][pitch]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -758,7 +762,8 @@ __global__ void __launch_bounds__(256) k_cggi_keyswitch(uint32_t* __restrict__ o
     const int j_begin = blockIdx.z * j_share;
     const int j_end = j_begin + j_share < Nin ? j_begin + j_share : Nin;
     const int total = base_log * levels;
-    const uint32_t keep = total >= 32 ? 0xFFFFFFFFu : (1u << total) - 1u, field = (1u << base_log) - 1u;
+    const uint32_t keep = total >= 32 ? 0xFFFFFFFFu : (1u << total) - 1u;
+    const uint32_t field = base_log >= 32 ? 0xFFFFFFFFu : (1u << base_log) - 1u;
     uint32_t half_sum = 0;
     for (int l = 0; l < levels; ++l) half_sum += 1u << (base_log * l + base_log - 1);
     int acc[MT][4][4];
@@ -778,18 +783,27 @@ __global__ void __launch_bounds__(256) k_cggi_keyswitch(uint32_t* __restrict__ o
             uint32_t v = ok ? in[b * (Nin + 1) + j0 + jj] : 0u;
             v = total >= 32 ? v : (uint32_t)(((uint64_t)v + (1ULL << (31 - total))) >> (32 - total));
             v = (v + half_sum) & keep;
-            int8_t* d = dig + row * pitch + jj * levels;
-            for (int l = 0; l < levels; ++l)
-                d[l] = ok ? (int8_t)((int)((v >> (base_log * (levels - 1 - l))) & field) - (1 << (base_log - 1))) : 0;
+            int8_t* d = dig + row * pitch + jj * dj;
+            for (int l = 0; l < levels; ++l) {
+                const uint32_t x = ((v >> (base_log * (levels - 1 - l))) & field) - (1u << (base_log - 1));
+                if constexpr (PARTS == 1) {
+                    d[l] = ok ? (int8_t)(int)x : 0;
+                } else {
+                    const uint32_t y = x + (0x80808080u >> (8 * (4 - PARTS)));
+#pragma unroll
+                    for (int i = 0; i < PARTS; ++i)
+                        d[l * PARTS + i] = ok ? (int8_t)((int)((y >> (8 * i)) & 255u) - 128) : 0;
+                }
+            }
         }
         __syncthreads();
-        const long long k_rows = (long long)Nin * levels, k0 = (long long)j0 * levels;
+        const long long k_rows = (long long)Nin * dj, k0 = (long long)j0 * dj;
         for (int kk = 0; kk < kc; kk += 32) {
             uint32_t w[8];
 #pragma unroll
             for (int r = 0; r < 8; ++r) {
                 const long long kr = k0 + kk + (lane & 3) * 4 + (r & 3) + (r >> 2) * 16;
-                w[r] = col_ok && kr < k_rows ? __ldg(ksk + kr * (n + 1) + col) : 0u;
+                w[r] = col_ok && kr < k_rows ? __ldg(ksk + kr / PARTS * (n + 1) + col) << (8 * (int)(kr % PARTS)) : 0u;
             }
             uint32_t p0[4], p1[4];
             byte_planes(p0, w[0], w[1], w[2], w[3]);
@@ -916,13 +930,13 @@ struct ExtprodF {
     static int run(A... a) { return launch_extprod_t<LOGM, LEVELS>(a...); }
 };
 
-template <int MT>
+template <int MT, int PARTS>
 int launch_keyswitch_t(uint32_t* out, const uint32_t* in, long long B, const uint32_t* ksk, int N, int n, int base_log,
                        int levels, cudaStream_t st) {
-    const size_t smem = (size_t)32 * MT * (KS_J * levels + 16);
+    const size_t smem = (size_t)32 * MT * (KS_J * levels * PARTS + 16);
     if (smem > 48 * 1024) {
-        const int e = (int)cudaFuncSetAttribute(k_cggi_keyswitch<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                (int)smem);
+        const int e = (int)cudaFuncSetAttribute(k_cggi_keyswitch<MT, PARTS>,
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e) return e;
     }
     const long long cols = (n + 1 + KS_COLS - 1) / KS_COLS, rows = (B + 32 * MT - 1) / (32 * MT);
@@ -938,17 +952,28 @@ int launch_keyswitch_t(uint32_t* out, const uint32_t* in, long long B, const uin
         k_ks_body<<<(unsigned)blocks, 256, 0, st>>>(out, in, B, N, n);
         note_launch();
     }
-    k_cggi_keyswitch<MT><<<dim3((unsigned)cols, (unsigned)rows, (unsigned)shares), 256, smem, st>>>(
+    k_cggi_keyswitch<MT, PARTS><<<dim3((unsigned)cols, (unsigned)rows, (unsigned)shares), 256, smem, st>>>(
         out, in, B, ksk, N, n, base_log, levels, j_share);
     note_launch();
     return (int)cudaGetLastError();
 }
 
 // Warps take four 16-row tiles of ciphertexts where the batch fills them, one otherwise.
+template <int PARTS>
+int launch_keyswitch_p(uint32_t* out, const uint32_t* in, long long B, const uint32_t* ksk, int N, int n, int base_log,
+                       int levels, cudaStream_t st) {
+    return B > 32 ? launch_keyswitch_t<4, PARTS>(out, in, B, ksk, N, n, base_log, levels, st)
+                  : launch_keyswitch_t<1, PARTS>(out, in, B, ksk, N, n, base_log, levels, st);
+}
+
+// Bytes a digit takes: one up to 8 bits ([-128, 128) as it stands), else those that hold it
+// balanced, at most the word's four.
 int launch_keyswitch(uint32_t* out, const uint32_t* in, long long B, const uint32_t* ksk, int N, int n, int base_log,
                      int levels, cudaStream_t st) {
-    return B > 32 ? launch_keyswitch_t<4>(out, in, B, ksk, N, n, base_log, levels, st)
-                  : launch_keyswitch_t<1>(out, in, B, ksk, N, n, base_log, levels, st);
+    if (base_log <= 8) return launch_keyswitch_p<1>(out, in, B, ksk, N, n, base_log, levels, st);
+    if (base_log <= 15) return launch_keyswitch_p<2>(out, in, B, ksk, N, n, base_log, levels, st);
+    if (base_log <= 23) return launch_keyswitch_p<3>(out, in, B, ksk, N, n, base_log, levels, st);
+    return launch_keyswitch_p<4>(out, in, B, ksk, N, n, base_log, levels, st);
 }
 
 int launch_to_fourier(int N, double2* outp, const uint32_t* rows, long long count, const FourierTables* ft,
