@@ -105,16 +105,13 @@ bool transform_together(RNS_MLWE o, RNS_MLWE i, bool inverse, const char* where)
 }
 
 bool gadget_all_ok(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly);
-void gadget_mac_all(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly, int mode, const char* where);
+bool gadget_mac_all(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly, int mode, const char* where);
 
 // gadget_mul_{add,sub}to_polynomial (gadget.c:5-36): digit j = limb j of the
 // coefficient-domain `poly`, lifted to the key's extended limbs, transformed, and
-// multiplied into `out` with ksk[digit].
-void gadget_mac(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly, int mode, const char* where) {
-    if (gadget_all_ok(out, ksk, poly)) {
-        gadget_mac_all(out, ksk, poly, mode, where);
-        return;
-    }
+// multiplied into `out` with ksk[digit].  False: the product failed (the error is recorded).
+bool gadget_mac(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly, int mode, const char* where) {
+    if (gadget_all_ok(out, ksk, poly)) return gadget_mac_all(out, ksk, poly, mode, where);
     IncNtt* t = pool(out);
     Poly* tmp = poly_create(0, ksk[0]->b->rns_mask, reinterpret_cast<IncNtt*>(ksk[0]->b->ntt));
     uint64_t k = 0;
@@ -127,6 +124,7 @@ void gadget_mac(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly, int mode, const char* w
         op_product(P_(out->b), P_(key->b), tmp, mode, where);
     }
     poly_destroy(tmp);
+    return true;
 }
 
 void set_masks(RNS_MLWE m, uint64_t mask) {
@@ -289,8 +287,19 @@ bool gadget_all_ok(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly) {
     return true;
 }
 
+// Device scratch that goes back to the engine's pool with its scope (kernels already enqueued
+// on the engine stream finish before the block's next user on that stream).
+struct DeviceScratch {
+    void* p;
+    explicit DeviceScratch(size_t bytes) : p(device_alloc(bytes)) {}
+    ~DeviceScratch() { device_free(p); }
+    DeviceScratch(const DeviceScratch&) = delete;
+    DeviceScratch& operator=(const DeviceScratch&) = delete;
+};
+
 // Digit polynomials of `poly` times the keys into out's extended limbs (mode as GadgetMac).
-void gadget_mac_all(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly, int mode, const char* where) {
+// False: a launch or the scratch failed, the error is recorded and out's rows are undefined.
+bool gadget_mac_all(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly, int mode, const char* where) {
     IncNtt* t = pool(out);
     const long long N = (long long)t->pub.N;
     const uint64_t ext = ksk[0]->b->rns_mask;
@@ -308,8 +317,9 @@ void gadget_mac_all(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly, int mode, const cha
     int per = (int)(kGadgetScratch / ((size_t)gm.ne * N * 8));
     if (per < 1) per = 1;
     if (per > nd) per = nd;
-    uint64_t* D = (uint64_t*)device_alloc((size_t)per * gm.ne * N * 8);
-    if (!D) return;
+    const DeviceScratch scratch((size_t)per * gm.ne * N * 8);
+    uint64_t* D = (uint64_t*)scratch.p;
+    if (!D) return false;
     for (int j0 = 0; j0 < nd;) {
         // consecutive limbs are rows N apart
         int n = 1;
@@ -339,10 +349,10 @@ void gadget_mac_all(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly, int mode, const cha
                     one.in[i] = poly->pub.coeffs[dig[j0 + d]];
                     one.out[i] = rs.out[i] + d * rs.digit_stride;
                 }
-                if (!check_cuda(launch_ntt(one, t->d_info, false, stream()), where)) return;
+                if (!check_cuda(launch_ntt(one, t->d_info, false, stream()), where)) return false;
             }
         } else if (!check_cuda(launch_ntt(rs, t->d_info, false, stream()), where)) {
-            return;
+            return false;
         }
         for (int d = 0; d < n; ++d)
             for (int c = 0; c < comps; ++c) {
@@ -355,15 +365,14 @@ void gadget_mac_all(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly, int mode, const cha
         const int e = comps == 2   ? launch_gadget_mac<2>(gm, D, t->d_info, N, S)
                       : comps == 3 ? launch_gadget_mac<3>(gm, D, t->d_info, N, S)
                                    : launch_gadget_mac<4>(gm, D, t->d_info, N, S);
-        if (!check_cuda(e, where)) return;
+        if (!check_cuda(e, where)) return false;
         if (mode == 0) mode = 1;
         if (mode == 3) mode = 2;
         j0 += n;
     }
     set_masks(out, ext);
-    device_free(D);
+    return true;
 }
-
 
 // Gaussian integers (truncated Box-Muller draws), four per ChaCha20 block from ctr on.
 __global__ void k_gauss_int(int64_t* out, long long n, double sigma, const __grid_constant__ PrngKey key,
@@ -997,15 +1006,21 @@ void mlwe_RNSc_GHS_hybrid_keyswitch(void* out, void* in, void* ksk, uint64_t lvl
     const uint64_t divide_mask = extended & ~i->b->rns_mask;
     set_masks(o, extended);
     uint64_t first = c0;
+    bool ok = true;
     if (gadget_all_ok(o, K[c0], P_(i->a[c0]))) {  // writes every extended row: only the others are zeroed
         zero_mlwe(o, vc_where_, ~extended);
-        gadget_mac_all(o, K[c0], P_(i->a[c0]), 3, vc_where_);
+        ok = gadget_mac_all(o, K[c0], P_(i->a[c0]), 3, vc_where_);
         first = c0 + 1;
     } else {
         zero_mlwe(o, vc_where_);
     }
-    for (uint64_t k = first; k < i->r; ++k)
-        if (K[k] != nullptr) gadget_mac(o, K[k], P_(i->a[k]), 2, vc_where_);
+    for (uint64_t k = first; k < i->r && ok; ++k)
+        if (K[k] != nullptr) ok = gadget_mac(o, K[k], P_(i->a[k]), 2, vc_where_);
+    if (!ok) {  // no stale rows in the result of a failed call
+        zero_mlwe(o, vc_where_);
+        VC_FINISH();
+        return;
+    }
     mlwe_RNS_to_RNSc(o, o);
     mlwe_round_division_RNSc(o, divide_mask);
     uint64_t keep = 0;
@@ -1133,15 +1148,21 @@ void mgsw_external_product(void* out, void* mgsw, void* in, uint64_t ell, uint64
     const uint64_t extended = G[0]->b->rns_mask;
     set_masks(o, extended);
     uint64_t first = 0;
+    bool ok = true;
     if (r > 0 && o != i && gadget_all_ok(o, G, P_(i->a[0]))) {
         zero_mlwe(o, vc_where_, ~extended);
-        gadget_mac_all(o, G, P_(i->a[0]), 0, vc_where_);
+        ok = gadget_mac_all(o, G, P_(i->a[0]), 0, vc_where_);
         first = 1;
     } else {
         zero_mlwe(o, vc_where_);
     }
-    for (uint64_t j = first; j < r; ++j) gadget_mac(o, &G[j * ell], P_(i->a[j]), 1, vc_where_);
-    gadget_mac(o, &G[r * ell], P_(i->b), 1, vc_where_);
+    for (uint64_t j = first; j < r && ok; ++j) ok = gadget_mac(o, &G[j * ell], P_(i->a[j]), 1, vc_where_);
+    ok = ok && gadget_mac(o, &G[r * ell], P_(i->b), 1, vc_where_);
+    if (!ok) {
+        zero_mlwe(o, vc_where_);
+        VC_FINISH();
+        return;
+    }
     if (special_primes > 0) {
         mlwe_RNS_to_RNSc(o, o);
         uint64_t divide_mask = 0, count = 0;
