@@ -3,7 +3,13 @@
 // device: no kernel of it may start.
 //
 //   gadget_host <entry> <case>     prints the engine calls the entry point made
+#include <cuda_runtime.h>
+
+// kernel launches report what the case asks for (without a device none of them starts)
+static cudaError_t fake_last_error();
+#define cudaGetLastError fake_last_error
 #include "../vfhe_b200/csrc/abi_mlwe.cu"
+#undef cudaGetLastError
 
 #include <stdio.h>
 #include <stdlib.h>
@@ -16,6 +22,8 @@ std::string g_case;
 std::map<std::string, int> g_calls;
 void call(const char* name) { ++g_calls[name]; }
 }  // namespace
+
+static cudaError_t fake_last_error() { return g_case == "launch_fails" ? cudaErrorInvalidValue : cudaSuccess; }
 
 namespace vc {
 Context& ctx() {
@@ -100,6 +108,13 @@ int main(int argc, char** argv) {
         t.info[1].fp64 = 0;
         for (auto& k : key) k->a[0]->rns_mask = k->b->rns_mask = 0b1101;
     }
+    // operands that share a polynomial
+    if (g_case == "key_mask_is_output_body") key[1]->a[0] = out->b;
+    if (g_case == "key_body_is_output_mask") key[2]->b = out->a[0];
+    if (g_case == "output_mask_is_output_body") out->a[0] = out->b;
+    if (g_case == "input_body_is_output_mask") in->b = out->a[0];
+    if (g_case == "input_body_is_output_body") in->b = out->b;
+    if (g_case == "input_mask_is_output_body") in->a[0] = out->b;
     if (entry == "keyswitch") {
         void* comp[1] = {key};
         mlwe_RNSc_GHS_hybrid_keyswitch(out, in, comp, 0);

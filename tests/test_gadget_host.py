@@ -33,8 +33,8 @@ def calls(tmp_path_factory):
 @pytest.mark.parametrize("entry", ["keyswitch", "external_product"])
 @pytest.mark.parametrize("case", ["transform_fails", "launch_fails", "no_scratch"])
 def test_a_failed_product_gives_its_scratch_back_and_stops(calls, entry, case):
-    """(launch_fails: without a device the product's kernel cannot launch.)  The output is
-    neither divided nor added to; its extended rows are zeroed instead of left as they were."""
+    """The output is neither divided nor added to; its extended rows are zeroed instead of left
+    as they were."""
     got = calls(entry, case)
     assert got["error"] >= 1
     assert got.get("alloc", 0) == got.get("free", 0) == (0 if case == "no_scratch" else 1)
@@ -46,3 +46,23 @@ def test_a_failed_product_gives_its_scratch_back_and_stops(calls, entry, case):
 def test_a_large_digit_outside_the_key_goes_digit_by_digit(calls, entry):
     got = calls(entry, "large_digit")
     assert "alloc" not in got and got["product"] >= 6
+
+
+@pytest.mark.parametrize("entry,case", [
+    ("keyswitch", "key_mask_is_output_body"), ("keyswitch", "key_body_is_output_mask"),
+    ("keyswitch", "output_mask_is_output_body"), ("keyswitch", "input_mask_is_output_body"),
+    ("external_product", "key_mask_is_output_body"), ("external_product", "key_body_is_output_mask"),
+    ("external_product", "output_mask_is_output_body"), ("external_product", "input_mask_is_output_body"),
+    ("external_product", "input_body_is_output_mask"), ("external_product", "input_body_is_output_body")])
+def test_shared_polynomials_go_digit_by_digit(calls, entry, case):
+    """The output is zeroed before an input is read, and the product whose operands share a
+    polynomial (3 digits, 2 components) is taken one digit and component after the other."""
+    got = calls(entry, case)
+    assert got["zero"] == 1 and got["product"] >= 6
+
+
+@pytest.mark.parametrize("entry", ["keyswitch", "external_product"])
+def test_separate_polynomials_take_every_digit_at_once(calls, entry):
+    got = calls(entry, "plain")
+    assert got["alloc"] == got["free"] == (1 if entry == "keyswitch" else 2)
+    assert "product" not in got and "error" not in got and got["divide"] == 1

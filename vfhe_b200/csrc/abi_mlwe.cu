@@ -256,7 +256,7 @@ int launch_gadget_mac(const GadgetMac& gm, const uint64_t* D, const PrimeInfo* p
 
 // Whether gadget_mac_all takes these operands: one pool, FP64 primes (the digits' own too: a
 // digit is read as a double before it is reduced), every key polynomial active at the same
-// extended limbs, blocks apart from one another and the digits.
+// extended limbs, and no output that is also the digits', a key's or another output's polynomial.
 bool gadget_all_ok(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly) {
     IncNtt* t = pool(out);
     const uint64_t ext = ksk[0]->b->rns_mask, mask = poly->pub.rns_mask;
@@ -274,17 +274,33 @@ bool gadget_all_ok(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly) {
     for (int j = 0, n = mask_indices(mask, t->pub.l, dig); j < n; ++j)
         if (!t->info[dig[j]].fp64) return false;
     if (ne == 0 || t->logP < 8 || t->logP > 17) return false;
+    Poly* o[kGadgetComps];
     for (int c = 0; c < comps; ++c) {
-        Poly* o = P_(c < (int)out->r ? out->a[c] : out->b);
-        if (!covers(o, ext) || o == poly) return false;
-        for (int j = 0; j < nd; ++j) {
-            RNS_MLWE k = ksk[j];
-            if (!k || (int)k->r + 1 != comps) return false;
+        o[c] = P_(c < (int)out->r ? out->a[c] : out->b);
+        if (!covers(o[c], ext) || o[c] == poly) return false;
+        for (int d = 0; d < c; ++d)
+            if (o[c] == o[d]) return false;
+    }
+    for (int j = 0; j < nd; ++j) {
+        RNS_MLWE k = ksk[j];
+        if (!k || (int)k->r + 1 != comps) return false;
+        for (int c = 0; c < comps; ++c) {
             Poly* kp = P_(c < (int)k->r ? k->a[c] : k->b);
-            if (!covers(kp, ext) || kp->pub.rns_mask != ext || kp == o) return false;
+            if (!covers(kp, ext) || kp->pub.rns_mask != ext) return false;
+            for (int d = 0; d < comps; ++d)
+                if (kp == o[d]) return false;
         }
     }
     return true;
+}
+
+// Whether a polynomial belongs to both samples: the one written is then zeroed before the
+// other is read (mlwe.c:557-598, mgsw.c:6-72), so the first product may not write it instead.
+bool share_polynomials(RNS_MLWE a, RNS_MLWE b) {
+    for (uint64_t i = 0; i <= a->r; ++i)
+        for (uint64_t j = 0; j <= b->r; ++j)
+            if ((i < a->r ? a->a[i] : a->b) == (j < b->r ? b->a[j] : b->b)) return true;
+    return false;
 }
 
 // Device scratch that goes back to the engine's pool with its scope (kernels already enqueued
@@ -1007,7 +1023,7 @@ void mlwe_RNSc_GHS_hybrid_keyswitch(void* out, void* in, void* ksk, uint64_t lvl
     set_masks(o, extended);
     uint64_t first = c0;
     bool ok = true;
-    if (gadget_all_ok(o, K[c0], P_(i->a[c0]))) {  // writes every extended row: only the others are zeroed
+    if (!share_polynomials(o, i) && gadget_all_ok(o, K[c0], P_(i->a[c0]))) {  // writes every extended row: only the others are zeroed
         zero_mlwe(o, vc_where_, ~extended);
         ok = gadget_mac_all(o, K[c0], P_(i->a[c0]), 3, vc_where_);
         first = c0 + 1;
@@ -1149,7 +1165,7 @@ void mgsw_external_product(void* out, void* mgsw, void* in, uint64_t ell, uint64
     set_masks(o, extended);
     uint64_t first = 0;
     bool ok = true;
-    if (r > 0 && o != i && gadget_all_ok(o, G, P_(i->a[0]))) {
+    if (r > 0 && !share_polynomials(o, i) && gadget_all_ok(o, G, P_(i->a[0]))) {
         zero_mlwe(o, vc_where_, ~extended);
         ok = gadget_mac_all(o, G, P_(i->a[0]), 0, vc_where_);
         first = 1;
