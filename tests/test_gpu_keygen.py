@@ -287,3 +287,30 @@ def test_key_files_save_load_use(cuda, tmp_path):
     tv = to_device32(test_vector(lut, p))
     lwe = to_device32(keys.encrypt(rng.integers(0, p.t, 256), rng))
     assert torch.equal(dev1.bootstrap(lwe, tv), dev2.bootstrap(lwe, tv))
+
+
+@pytest.mark.parametrize("N", [512, 2048])
+def test_torus_device_keys_at_every_ring_degree(cuda, N):
+    """Bootstrapping-key rows of the smallest and largest ring decrypt to their gadget message
+    within 8 sigma (the largest has more coefficients than a block has threads)."""
+    import torch
+
+    from vfhe_b200.cggi_fft import TorusParams, generate_device_keys, negacyclic_times_binary
+
+    p = TorusParams(n=3, N=N)
+    keys = generate_device_keys(p, np.random.default_rng(N), cuda)
+    torch.cuda.synchronize()
+    bsk = keys.bsk_d.cpu().numpy().view(np.uint32)
+    a, b = bsk[:, :, 0].copy(), bsk[:, :, 1].astype(np.int64)
+    for i in range(p.n):
+        for r in range(2 * p.bs_levels):
+            c, lv = divmod(r, p.bs_levels)
+            m = int(keys.s[i]) << (32 - p.bs_base_log * (lv + 1))
+            if c == 0:
+                a[i, r, 0] = (int(a[i, r, 0]) - m) & 0xFFFFFFFF
+            else:
+                b[i, r, 0] -= m
+    e = (b - negacyclic_times_binary(a, keys.S).astype(np.int64)) & 0xFFFFFFFF
+    e = np.where(e >= 1 << 31, e - (1 << 32), e)
+    assert np.abs(e).max() <= 8 * p.glwe_sigma * 2**32
+    assert np.abs(e).max() > 0 and len(np.unique(a)) > a.size // 2

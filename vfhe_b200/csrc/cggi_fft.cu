@@ -1019,41 +1019,49 @@ __device__ __forceinline__ int32_t torus_gauss(const PrngKey& key, uint64_t coun
     return (int32_t)(int64_t)llrint(sigma32 * sqrt(-2.0 * log(u1)) * cospi(2.0 * u2));
 }
 
-// one CTA of N threads per bootstrapping-key row; thread k computes coefficient k
-__global__ void k_torus_bsk_rows(uint32_t* __restrict__ rows, const int32_t* __restrict__ s,
-                                 const int32_t* __restrict__ S, int N, int levels, int base_log, double sigma32,
-                                 const __grid_constant__ PrngKey key, uint64_t u0, uint64_t g0) {
+// One CTA per bootstrapping-key row, its threads over the coefficients k (N = 2048 has more of
+// them than a CTA has threads).
+constexpr int kBskThreads = 1024;
+
+__global__ void __launch_bounds__(kBskThreads) k_torus_bsk_rows(uint32_t* __restrict__ rows, const int32_t* __restrict__ s,
+                                                                const int32_t* __restrict__ S, int N, int levels,
+                                                                int base_log, double sigma32,
+                                                                const __grid_constant__ PrngKey key, uint64_t u0,
+                                                                uint64_t g0) {
     extern __shared__ uint32_t tsm[];  // a [N], S [N]
     uint32_t* a = tsm;
     uint32_t* Ssh = tsm + N;
     const long long row = blockIdx.x;  // i * 2 levels + r
     const int i = (int)(row / (2 * levels)), r = (int)(row - (long long)i * 2 * levels);
-    const int k = threadIdx.x;
     const uint64_t per_row = (uint64_t)(N / 16);
-    if ((k & 15) == 0) {
-        uint32_t blk[16];
-        chacha20_block(key, u0 + (uint64_t)row * per_row + (uint64_t)(k >> 4), kStreamUniform, blk);
+    for (int k = threadIdx.x; k < N; k += blockDim.x) {
+        if ((k & 15) == 0) {
+            uint32_t blk[16];
+            chacha20_block(key, u0 + (uint64_t)row * per_row + (uint64_t)(k >> 4), kStreamUniform, blk);
 #pragma unroll
-        for (int w = 0; w < 16; ++w) a[k + w] = blk[w];
+            for (int w = 0; w < 16; ++w) a[k + w] = blk[w];
+        }
+        Ssh[k] = (uint32_t)S[k];
     }
-    Ssh[k] = (uint32_t)S[k];
     __syncthreads();
-    // (a S)_k = sum_j a_j S_(k-j) with the sign of the wrap (X^N = -1)
-    uint32_t acc = 0;  // products mod 2^32: a small signed key entry multiplies as its residue
-    for (int j = 0; j <= k; ++j) acc += a[j] * Ssh[k - j];
-    for (int j = k + 1; j < N; ++j) acc -= a[j] * Ssh[k - j + N];
-    const int32_t e = torus_gauss(key, g0 + (uint64_t)row * (uint64_t)(N / 4) + (uint64_t)(k >> 2), k, sigma32);
-    uint32_t b = acc + (uint32_t)e;
-    uint32_t av = a[k];
     const int c = r / levels, l = r - c * levels;
-    if (k == 0) {
-        const uint32_t m = (uint32_t)s[i] << (32 - base_log * (l + 1));
-        if (c == 0) av += m;
-        else b += m;
-    }
     uint32_t* out = rows + (size_t)row * 2 * N;
-    out[k] = av;
-    out[N + k] = b;
+    for (int k = threadIdx.x; k < N; k += blockDim.x) {
+        // (a S)_k = sum_j a_j S_(k-j) with the sign of the wrap (X^N = -1)
+        uint32_t acc = 0;  // products mod 2^32: a small signed key entry multiplies as its residue
+        for (int j = 0; j <= k; ++j) acc += a[j] * Ssh[k - j];
+        for (int j = k + 1; j < N; ++j) acc -= a[j] * Ssh[k - j + N];
+        const int32_t e = torus_gauss(key, g0 + (uint64_t)row * (uint64_t)(N / 4) + (uint64_t)(k >> 2), k, sigma32);
+        uint32_t b = acc + (uint32_t)e;
+        uint32_t av = a[k];
+        if (k == 0) {
+            const uint32_t m = (uint32_t)s[i] << (32 - base_log * (l + 1));
+            if (c == 0) av += m;
+            else b += m;
+        }
+        out[k] = av;
+        out[N + k] = b;
+    }
 }
 
 // one thread per key-switching-key row (j, l): mask, then body
@@ -1167,7 +1175,7 @@ int vfhe_cuda_cggi_fft_gen_keys(uint32_t* d_bsk_rows, uint32_t* d_ksk, const int
     const uint64_t u0 = prng_advance(bsk_rows * (N / 16) + ksk_rows * ((n + 15) / 16));
     const uint64_t g0 = prng_advance(bsk_rows * (N / 4) + ksk_rows);
     const PrngKey key = prng_key();
-    k_torus_bsk_rows<<<(unsigned)bsk_rows, N, 2 * N * sizeof(uint32_t), st>>>(
+    k_torus_bsk_rows<<<(unsigned)bsk_rows, N < kBskThreads ? N : kBskThreads, 2 * N * sizeof(uint32_t), st>>>(
         d_bsk_rows, d_s, d_S, (int)N, (int)bs_levels, (int)bs_base_log, glwe_sigma * 4294967296.0, key, u0, g0);
     note_launch();
     if (!check_cuda(cudaGetLastError(), where)) return 1;
