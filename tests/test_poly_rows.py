@@ -1,0 +1,46 @@
+"""Reading a polynomial's rows: into an array the caller gives, on both engines, and through
+vfhe_cuda_poly_read_rows."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+N, SIZES = 64, [50, 40, 45]
+
+
+def _poly(engine):
+    from vfhe_b200.arith import Polynomial, Ring
+
+    ring = Ring(N, prime_size=SIZES, split_degree=1, engine=engine)
+    p = Polynomial(ring)
+    rng = np.random.default_rng(3)
+    rows = np.stack([rng.integers(0, q, N, dtype=np.uint64) for q in ring.primes])
+    p.set_rows(rows)
+    return p, rows
+
+
+def _given_arrays(engine):
+    p, rows = _poly(engine)
+    out = np.zeros((len(SIZES) + 1, N), dtype=np.uint64)
+    assert p.rows(out) is out
+    assert np.array_equal(out[:-1], rows) and not out[-1].any()
+    signed = np.zeros((len(SIZES), N), dtype=np.int64)
+    assert np.array_equal(p.rows(signed).view(np.uint64), rows)
+    locked = np.zeros((len(SIZES), N), dtype=np.uint64)
+    locked.flags.writeable = False
+    for bad in (np.zeros((len(SIZES) - 1, N), dtype=np.uint64), np.zeros(len(SIZES) * N - 1, dtype=np.uint64),
+                np.zeros((len(SIZES), 2 * N), dtype=np.uint64)[:, ::2], np.zeros((len(SIZES), N), dtype=np.uint32),
+                locked):
+        with pytest.raises(ValueError):
+            p.rows(bad)
+        assert not bad.any()
+
+
+def test_rows_into_a_given_array(oracle_engine):
+    _given_arrays(oracle_engine)
+
+
+@pytest.mark.gpu
+def test_rows_into_a_given_array_cuda(cuda):
+    _given_arrays(cuda)

@@ -455,18 +455,23 @@ class Polynomial:
 
     # -- coefficient IO
     def rows(self, out: np.ndarray | None = None) -> np.ndarray:
-        """Raw rows of the ring's limbs, [ell][N] uint64, in the engine's row layout (into
-        ``out``, contiguous, when given)."""
+        """Raw rows of the ring's limbs, [ell][N] uint64, in the engine's row layout (into the
+        first ell N words of ``out``, contiguous 64-bit integers, when given)."""
         eng, idx = self.ring.engine, self.ring.prime_indices
+        words = len(idx) * self.ring.N
         if out is None:
             out = np.empty((len(idx), self.ring.N), dtype=np.uint64)
+        elif out.dtype not in (np.uint64, np.int64) or not out.flags.c_contiguous or not out.flags.writeable \
+                or out.size < words:
+            raise ValueError(f"rows need a writable contiguous array of at least {words} 64-bit integers")
         if eng.name == "cuda":
             self._lib.vfhe_cuda_poly_read_rows(self.obj, self.ring.ffi.from_buffer("uint64_t[]", out),
                                                self.ring.ffi.new("uint32_t[]", idx), len(idx))
             self._chk("vfhe_cuda_poly_read_rows")
         else:
+            flat = out.reshape(-1)
             for k, i in enumerate(idx):
-                out[k] = self.row(i)
+                flat[k * self.ring.N:(k + 1) * self.ring.N] = self.row(i)
         return out
 
     def set_rows(self, rows: np.ndarray) -> None:
