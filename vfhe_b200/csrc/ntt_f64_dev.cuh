@@ -57,6 +57,9 @@ __device__ __forceinline__ int lane_tw_index(int g, int b, int h) {
     return (((g >> 5) * 15 + ((1 << (3 - b)) - 1) + h) << 5) + (g & 31);
 }
 
+// How a kernel wants its tiles' addresses: see fput_at.
+enum TileForm { kStraight, kLooped };
+
 // Stages of a tile's pass at bit 0 (the forward transform's last, the inverse's first): the
 // others take four each.
 template <int K>
@@ -185,7 +188,13 @@ __device__ __forceinline__ void edge_tw(double2* w, int b, int t, int hi, int lo
     }
 }
 
-template <int K, int LO, int BHI, int BLO>
+// Whether a tile's exchange and forward twiddle addresses are left to the compiler: see fput_at.
+template <int K, TileForm F>
+__host__ __device__ constexpr bool whole_addresses() {
+    return EdgePass<K>::NST == 4 && F == kStraight;
+}
+
+template <int K, int LO, int BHI, int BLO, TileForm F = kStraight>
 __device__ __forceinline__ void f_fwd_tw(PassTw<LO, BHI, BLO>& T, int t, int hi, int logP, const FCtx& c) {
 #pragma unroll
     for (int b = BHI; b >= BLO; --b) {
@@ -198,7 +207,7 @@ __device__ __forceinline__ void f_fwd_tw(PassTw<LO, BHI, BLO>& T, int t, int hi,
 #pragma unroll
             for (int h = 0; h < (1 << (3 - bb)); ++h)
                 T.w[PassTw<LO, BHI, BLO>::offset(b) + h] = __ldg(&c.mt[lane_tw_index(g, bb, h)]);
-        } else if constexpr (EdgePass<K>::NST == 4) {
+        } else if constexpr (whole_addresses<K, F>()) {
             const double2* p = c.tw + (1 << (logP - 1 - b)) + (hi << (K - b - 1));
 #pragma unroll
             for (int h = 0; h < (1 << (3 - bb)); ++h)
@@ -305,11 +314,15 @@ __host__ __device__ __forceinline__ constexpr int slot_step(int m) {
 }
 
 // Tiles whose passes all have four stages (2^8, 2^12) leave these addresses, and the forward
-// twiddles', to the compiler: with the split form their forward launches ran 6% longer (2400
-// rows of 2^12: 65.6 us split, 59.3 so; 9600 rows 212), the other tiles' shorter.
-template <int K, int LO>
+// twiddles', to the compiler where a kernel's tile code stands alone: with the split form their
+// forward launches ran 6% longer (2400 rows of 2^12: 65.6 us split, 59.3 so; 9600 rows 212),
+// the other tiles' shorter.  Kernels that walk tiles in a loop (kLooped) split them all the
+// same: whole addresses spill there (bytes a thread, whole and split: the work list's forward
+// kernel 692 and 268, 2^12 tiles in persistent grids 464 and 0, in the dataflow kernel 292 and
+// 16; 2400 rows of 2^12 forward on one CTA an SM 145 us and 102).
+template <int K, int LO, TileForm F = kStraight>
 __device__ __forceinline__ void fput_at(double* sm, const double (&x)[16], int t) {
-    if constexpr (EdgePass<K>::NST == 4) {
+    if constexpr (whole_addresses<K, F>()) {
 #pragma unroll
         for (int m = 0; m < 16; ++m) sm[pad(own<LO>(t, m))] = x[m];
         return;
@@ -319,9 +332,9 @@ __device__ __forceinline__ void fput_at(double* sm, const double (&x)[16], int t
     for (int m = 0; m < 16; ++m) p[slot_step<K, LO>(m)] = x[m];
 }
 
-template <int K, int LO>
+template <int K, int LO, TileForm F = kStraight>
 __device__ __forceinline__ void fget_at(double (&x)[16], const double* sm, int t) {
-    if constexpr (EdgePass<K>::NST == 4) {
+    if constexpr (whole_addresses<K, F>()) {
 #pragma unroll
         for (int m = 0; m < 16; ++m) x[m] = sm[pad(own<LO>(t, m))];
         return;
@@ -437,7 +450,7 @@ __device__ __forceinline__ FCtx fwd_ctx(const PrimeInfo& pi) {
 // The forward passes of one tile whose 16 residues per thread are in x (x[m] at index
 // own<K - 4>(t, m), |x| <= q), the first pass's twiddles in tw1.  On return x[m] is at
 // index edge<K>(t, m) (|x| < 2^51, not reduced).
-template <int K, bool GROUP>
+template <int K, bool GROUP, TileForm F = kStraight>
 __device__ __forceinline__ void tile_fwd_passes(const FCtx& c, int logP, int hi, double* sm, int t, double (&x)[16],
                                                 const PassTw<K - 4, K - 1, K - 4>& tw1, int grp) {
     constexpr int L1 = K - 4;
@@ -445,26 +458,26 @@ __device__ __forceinline__ void tile_fwd_passes(const FCtx& c, int logP, int hi,
     constexpr int L3 = (K - 12) > 0 ? (K - 12) : 0;
     f_fwd_bits<K, L1, K - 1, L1>(x, tw1, c);
     PassTw<L2, L1 - 1, L2> tw2;
-    f_fwd_tw<K, L2, L1 - 1, L2>(tw2, t, hi, logP, c);
-    fput_at<K, L1>(sm, x, t);
+    f_fwd_tw<K, L2, L1 - 1, L2, F>(tw2, t, hi, logP, c);
+    fput_at<K, L1, F>(sm, x, t);
     tile_sync<K, GROUP>(grp);
-    fget_at<K, L2>(x, sm, t);
+    fget_at<K, L2, F>(x, sm, t);
     f_fwd_bits<K, L2, L1 - 1, L2>(x, tw2, c);
     if constexpr (L2 > 0) {
         PassTw<L3, L2 - 1, L3> tw3;
-        f_fwd_tw<K, L3, L2 - 1, L3>(tw3, t, hi, logP, c);
+        f_fwd_tw<K, L3, L2 - 1, L3, F>(tw3, t, hi, logP, c);
         tile_sync<K, GROUP>(grp);
-        fput_at<K, L2>(sm, x, t);
+        fput_at<K, L2, F>(sm, x, t);
         tile_sync<K, GROUP>(grp);
-        fget_at<K, L3>(x, sm, t);
+        fget_at<K, L3, F>(x, sm, t);
         f_fwd_bits<K, L3, L2 - 1, L3>(x, tw3, c);
         if constexpr (L3 > 0) {
             PassTw<0, L3 - 1, 0> tw4;
-            f_fwd_tw<K, 0, L3 - 1, 0>(tw4, t, hi, logP, c);
+            f_fwd_tw<K, 0, L3 - 1, 0, F>(tw4, t, hi, logP, c);
             tile_sync<K, GROUP>(grp);
-            fput_at<K, L3>(sm, x, t);
+            fput_at<K, L3, F>(sm, x, t);
             tile_sync<K, GROUP>(grp);
-            fget_at<K, 0>(x, sm, t);
+            fget_at<K, 0, F>(x, sm, t);
             f_fwd_bits<K, 0, L3 - 1, 0>(x, tw4, c);
         }
     }
@@ -478,7 +491,7 @@ __device__ __forceinline__ void tile_fwd_passes(const FCtx& c, int logP, int hi,
 // when `store` is set (a thread whose tile only pads out a group computes without
 // storing).  GROUP, grp: the tile's threads synchronise at named barrier 1 + grp
 // (tile_sync).
-template <int K, bool IN_D, bool STAGED, bool GROUP = false>
+template <int K, bool IN_D, bool STAGED, bool GROUP = false, TileForm F = kStraight>
 __device__ __forceinline__ void tile_fwd_regs(const Tile& r, int logP, bool red, double* sm, int t, double (&x)[16],
                                               int grp = 0) {
     const FCtx c = fwd_ctx(*r.pi);
@@ -488,7 +501,7 @@ __device__ __forceinline__ void tile_fwd_regs(const Tile& r, int logP, bool red,
     // each pass's twiddles are requested before the exchange that precedes the pass,
     // so their latency overlaps the barrier
     PassTw<L1, K - 1, L1> tw1;
-    f_fwd_tw<K, L1, K - 1, L1>(tw1, t, hi, logP, c);
+    f_fwd_tw<K, L1, K - 1, L1, F>(tw1, t, hi, logP, c);
     if (STAGED) {
         const uint64_t* staged = reinterpret_cast<const uint64_t*>(sm);
 #pragma unroll
@@ -498,37 +511,37 @@ __device__ __forceinline__ void tile_fwd_regs(const Tile& r, int logP, bool red,
 #pragma unroll
         for (int m = 0; m < 16; ++m) x[m] = load_in(r.src + own<L1>(t, m), IN_D, red, c);
     }
-    tile_fwd_passes<K, GROUP>(c, logP, hi, sm, t, x, tw1, grp);
+    tile_fwd_passes<K, GROUP, F>(c, logP, hi, sm, t, x, tw1, grp);
 }
 
-template <int K, bool IN_D, bool STAGED, bool GROUP = false>
+template <int K, bool IN_D, bool STAGED, bool GROUP = false, TileForm F = kStraight>
 __device__ __forceinline__ void tile_fwd_one(const Tile& r, const RowSet& rows, double* sm, int t, bool store,
                                              int grp = 0) {
     double x[16];
-    tile_fwd_regs<K, IN_D, STAGED, GROUP>(r, rows.logP, rows.reduce_input != 0, sm, t, x, grp);
+    tile_fwd_regs<K, IN_D, STAGED, GROUP, F>(r, rows.logP, rows.reduce_input != 0, sm, t, x, grp);
     if (store) store_edge_canonical<K>(r.dst, x, t, r.pi->qd, r.pi->qinv, r.pi->q);
 }
 
 // Passes of the inverse from bit LO up, four stages each, after the pass below left its
 // residues in layout PREV.
-template <int K, int PREV, int LO, bool FINAL, bool GROUP>
+template <int K, int PREV, int LO, bool FINAL, bool GROUP, TileForm F>
 __device__ __forceinline__ void tile_inv_passes(const PrimeInfo& pi, const FCtx& c, int logP, int hi, double* sm, int t,
                                                 double (&x)[16], int grp) {
     constexpr bool last = LO + 4 == K;
     PassTw<LO, LO, LO + 3> tw;
     f_inv_tw<K, LO, LO, LO + 3, FINAL && last>(tw, t, hi, logP, c);
     if (PREV > 0) tile_sync<K, GROUP>(grp);  // the previous exchange is read
-    fput_at<K, PREV>(sm, x, t);
+    fput_at<K, PREV, F>(sm, x, t);
     tile_sync<K, GROUP>(grp);
-    fget_at<K, LO>(x, sm, t);
+    fget_at<K, LO, F>(x, sm, t);
     f_inv_bits<K, LO, LO, LO + 3, FINAL && last>(x, tw, c, pi);
-    if constexpr (!last) tile_inv_passes<K, LO, LO + 4, FINAL, GROUP>(pi, c, logP, hi, sm, t, x, grp);
+    if constexpr (!last) tile_inv_passes<K, LO, LO + 4, FINAL, GROUP, F>(pi, c, logP, hi, sm, t, x, grp);
 }
 
 // Inverse passes of the low K bits of one tile whose 16 residues per thread t are in x
 // (x[m] at index edge<K>(t, m), |x| < q; the forward passes leave this layout).  FINAL
 // (K == logP): P^-1 folded in.  On return x[m] is at index own<K - 4>(t, m) of the tile.
-template <int K, bool FINAL, bool GROUP = false>
+template <int K, bool FINAL, bool GROUP = false, TileForm F = kStraight>
 __device__ __forceinline__ void tile_inv_regs(const PrimeInfo& pi, int logP, int hi, double* sm, int t,
                                               double (&x)[16], int grp = 0) {
     constexpr int NST = EdgePass<K>::NST;
@@ -541,13 +554,13 @@ __device__ __forceinline__ void tile_inv_regs(const PrimeInfo& pi, int logP, int
     PassTw<0, 0, NST - 1> tw1;
     f_inv_tw<K, 0, 0, NST - 1, false>(tw1, t, hi, logP, c);
     f_inv_bits<K, 0, 0, NST - 1, false>(x, tw1, c, pi);
-    tile_inv_passes<K, 0, NST, FINAL, GROUP>(pi, c, logP, hi, sm, t, x, grp);
+    tile_inv_passes<K, 0, NST, FINAL, GROUP, F>(pi, c, logP, hi, sm, t, x, grp);
 }
 
 // Inverse transform of the low K bits of tile r.  FINAL (K == logP): P^-1 folded in,
 // canonical output; otherwise centred doubles for the column pass.  STAGED and store as
 // for tile_fwd_one.
-template <int K, bool FINAL, bool STAGED, bool GROUP = false>
+template <int K, bool FINAL, bool STAGED, bool GROUP = false, TileForm F = kStraight>
 __device__ __forceinline__ void tile_inv_one(const Tile& r, const RowSet& rows, double* sm, int t, bool store,
                                              int grp = 0) {
     const PrimeInfo& pi = *r.pi;
@@ -564,7 +577,7 @@ __device__ __forceinline__ void tile_inv_one(const Tile& r, const RowSet& rows, 
         load_edge_u64<K>(x, r.src, t);
     }
     if (STAGED) tile_sync<K, GROUP>(grp);  // every input is in registers before the exchanges reuse the buffer
-    tile_inv_regs<K, FINAL, GROUP>(pi, rows.logP, r.hi, sm, t, x, grp);
+    tile_inv_regs<K, FINAL, GROUP, F>(pi, rows.logP, r.hi, sm, t, x, grp);
     constexpr int LAST = K - 4;
     if (!store) return;
 #pragma unroll
