@@ -32,6 +32,17 @@ struct ChainLimbs {
     uint32_t p[kMaxLimbs];  // pool index of each limb slot's prime
 };
 
+// Ring products take their tile addresses split at every size (2^12, 1200 rows: 82.0 us, 84.0
+// whole).  Blocks of 2^11 points in a split ring keep 16 consecutive residues a thread between
+// the transforms: the spectra stay in shared memory, so the coalesced edge pass saves no global
+// access, and its wide twiddle loads cost more there than its fewer bank conflicts give (us,
+// edge and linear: (11, 2) 192 rows 26.4 and 24.6, 1200 rows 102.4 and 98.4; (11, 4) 1200 rows
+// 221.4 and 216.9; but (10, 4) 95.8 and 101.5, (9, 2) 26.7 and 28.7, (11, 1) 40.9 and 43.0).
+template <int K, int S>
+constexpr TileForm chain_form() {
+    return K == 11 && S > 1 ? kLinear : kSplit;
+}
+
 // Up to 128 registers for 256-thread CTAs (two per SM, 70 KB of shared memory each at
 // N = 4096; a three-per-SM cap of 85 registers spilled 100-190 bytes per thread) and
 // 512-thread CTAs (N = 8192, 139 KB, one per SM); smaller CTAs are left to the compiler.
@@ -42,6 +53,7 @@ __global__ void __launch_bounds__(S << (K - 4), (S << (K - 4)) <= 256 ? 2 : 1) k
                                                           const PrimeInfo* __restrict__ primes, int nl) {
     constexpr int TPT = 1 << (K - 4), P = 1 << K, PADDED = P + (P >> 4);
     constexpr bool GROUP = S > 1;
+    constexpr TileForm F = chain_form<K, S>();
     extern __shared__ __align__(128) double csm[];
     double* spec = csm;            // [S][PADDED]: a's spectra, reduced, at pad(edge_base) + pad(edge_step)
     double* ex = csm + S * PADDED;  // [S][PADDED]: each block's exchanges, then b's spectra
@@ -53,7 +65,7 @@ __global__ void __launch_bounds__(S << (K - 4), (S << (K - 4)) <= 256 ? 2 : 1) k
     const double q = pi.qd, qinv = pi.qinv;
     const long long off = row * (long long)(S * P) + (long long)g * P;
     double* exg = ex + g * PADDED;
-    const int eb = edge_base<K>(t), pe = pad(eb);  // steps have bits that bases lack: pad adds up
+    const int eb = edge_base<K, F>(t), pe = pad(eb);  // steps have bits that bases lack: pad adds up
 
     Tile tile;
     tile.hi = 0;
@@ -62,9 +74,9 @@ __global__ void __launch_bounds__(S << (K - 4), (S << (K - 4)) <= 256 ? 2 : 1) k
     double x[16];
     // a's block g
     tile.src = a + off;
-    tile_fwd_regs<K, false, false, GROUP>(tile, K, false, exg, t, x, g);
+    tile_fwd_regs<K, false, false, GROUP, F>(tile, K, false, exg, t, x, g);
 #pragma unroll
-    for (int m = 0; m < 16; ++m) spec[g * PADDED + pe + pad(edge_step<K>(m))] = f_reduce(x[m], q, qinv);
+    for (int m = 0; m < 16; ++m) spec[g * PADDED + pe + pad(edge_step<K, F>(m))] = f_reduce(x[m], q, qinv);
     tile_sync<K, GROUP>(g);  // the block's last exchange reads are over before b's first write
     // b's block g.  Its twiddles are a's again; the prime's address goes through an
     // opaque move so that the compiler reloads them instead of keeping a's ~90 registers
@@ -73,23 +85,23 @@ __global__ void __launch_bounds__(S << (K - 4), (S << (K - 4)) <= 256 ? 2 : 1) k
     const PrimeInfo* pib;
     asm volatile("mov.b64 %0, %1;" : "=l"(pib) : "l"(&pi));
     tile.pi = pib;
-    tile_fwd_regs<K, false, false, GROUP>(tile, K, false, exg, t, x, g);
+    tile_fwd_regs<K, false, false, GROUP, F>(tile, K, false, exg, t, x, g);
     if constexpr (S == 1) {
         // pointwise: this thread's own slots of a's spectrum (written by this thread)
 #pragma unroll
         for (int m = 0; m < 16; ++m) {
             const double w = f_reduce(x[m], q, qinv);
-            x[m] = f_mulmod(spec[pe + pad(edge_step<K>(m))], w, __dmul_rn(w, qinv), q);  // |x| <= 3q/4
+            x[m] = f_mulmod(spec[pe + pad(edge_step<K, F>(m))], w, __dmul_rn(w, qinv), q);  // |x| <= 3q/4
         }
     } else {
         tile_sync<K, GROUP>(g);  // the block's exchanges are over: its buffer takes b's spectrum
 #pragma unroll
-        for (int m = 0; m < 16; ++m) exg[pe + pad(edge_step<K>(m))] = f_reduce(x[m], q, qinv);
+        for (int m = 0; m < 16; ++m) exg[pe + pad(edge_step<K, F>(m))] = f_reduce(x[m], q, qinv);
         __syncthreads();  // every block's spectra of a and b are in shared memory
         const ulonglong2* tw = reinterpret_cast<const ulonglong2*>(pi.twist) + eb;
 #pragma unroll
         for (int m = 0; m < 16; ++m) {
-            const int px = pe + pad(edge_step<K>(m));
+            const int px = pe + pad(edge_step<K, F>(m));
             double acc = 0.0, wrap = 0.0;
 #pragma unroll
             for (int i = 0; i < S; ++i) {
@@ -105,13 +117,13 @@ __global__ void __launch_bounds__(S << (K - 4), (S << (K - 4)) <= 256 ? 2 : 1) k
             // at most 8 terms of at most 3q/4 each: below 6q < 2^53
             acc = f_reduce(acc, q, qinv);
             wrap = f_reduce(wrap, q, qinv);
-            const uint64_t wi = tw[edge_step<K>(m)].x;
+            const uint64_t wi = tw[edge_step<K, F>(m)].x;
             const double wd = wi > pi.q / 2 ? (double)wi - q : (double)wi;
             x[m] = f_reduce(__dadd_rn(acc, f_mulmod(wrap, wd, __dmul_rn(wd, qinv), q)), q, qinv);
         }
         __syncthreads();  // every block's b spectrum is read before the exchanges reuse it
     }
-    tile_inv_regs<K, true, GROUP>(pi, K, 0, exg, t, x, g);
+    tile_inv_regs<K, true, GROUP, F>(pi, K, 0, exg, t, x, g);
     uint64_t* o = out + off;
 #pragma unroll
     for (int m = 0; m < 16; ++m) o[own<K - 4>(t, m)] = f_to_canonical(x[m], q, qinv, pi.q);

@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(TileThreads<K>::value, TileMinBlocks<K>::value
     }
     const long long tile = grp * tiles_per_cta + lt;
     const Tile r = locate<TABLE>(rows, primes, K, tile, tiles_per_row);
-    tile_fwd_one<K, IN_D, PERSIST, false, PERSIST ? kLooped : kStraight>(r, rows, sm, t, true);
+    tile_fwd_one<K, IN_D, PERSIST, false, PERSIST ? kSplit : kWhole>(r, rows, sm, t, true);
     if (!PERSIST) break;
     __syncthreads();  // the next trip rewrites shared memory
     }
@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(TileThreads<K>::value, TileMinBlocks<K>::value
     }
     const long long tile = grp * tiles_per_cta + lt;
     const Tile r = locate<TABLE>(rows, primes, K, tile, tiles_per_row);
-    tile_inv_one<K, FINAL, PERSIST, false, PERSIST ? kLooped : kStraight>(r, rows, sm, t, true);
+    tile_inv_one<K, FINAL, PERSIST, false, PERSIST ? kSplit : kWhole>(r, rows, sm, t, true);
     if (!PERSIST) break;
     __syncthreads();  // the next trip rewrites shared memory
     }

@@ -57,32 +57,36 @@ __device__ __forceinline__ int lane_tw_index(int g, int b, int h) {
     return (((g >> 5) * 15 + ((1 << (3 - b)) - 1) + h) << 5) + (g & 31);
 }
 
-// How a kernel wants its tiles' addresses: see fput_at.
-enum TileForm { kStraight, kLooped };
+// How a kernel wants its tiles' addresses and residues: kWhole and kSplit differ in the exchange
+// and twiddle addresses of tiles whose passes all have four stages (see fput_at); kLinear is
+// kSplit with 16 consecutive residues a thread at bit 0, for kernels that keep that pass's
+// residues in shared memory (chain.cu).
+enum TileForm { kWhole, kSplit, kLinear };
 
-// Stages of a tile's pass at bit 0 (the forward transform's last, the inverse's first): the
-// others take four each.
-template <int K>
+// Bits of the layout of a tile's pass at bit 0 (the forward transform's last, the inverse's
+// first), and its stages where the others take four each (kLinear: the forward pass takes the
+// stages left over, the inverse's last pass does).
+template <int K, TileForm F = kWhole>
 struct EdgePass {
-    static constexpr int NST = (K - 1) % 4 + 1;
+    static constexpr int NST = F == kLinear ? 4 : (K - 1) % 4 + 1;
 };
 
 // Residue m of thread t in the pass at bit 0: the pass's NST bits and the index's top 4 - NST
 // bits, so that neighbouring lanes own neighbouring groups of 2^NST residues and a warp's
 // global accesses are contiguous (16 consecutive residues a thread when NST = 4: lanes 128
 // bytes apart, 52 L1 wavefronts a 32-byte store against 8).
-template <int K>
+template <int K, TileForm F = kWhole>
 __device__ __forceinline__ int edge_base(int t) {
-    return t << EdgePass<K>::NST;
+    return t << EdgePass<K, F>::NST;
 }
-template <int K>
+template <int K, TileForm F = kWhole>
 __host__ __device__ __forceinline__ constexpr int edge_step(int m) {
-    constexpr int NST = EdgePass<K>::NST;
+    constexpr int NST = EdgePass<K, F>::NST;
     return ((m >> NST) << (K - 4 + NST)) | (m & ((1 << NST) - 1));
 }
-template <int K>
+template <int K, TileForm F = kWhole>
 __device__ __forceinline__ int edge(int t, int m) {
-    return edge_base<K>(t) + edge_step<K>(m);
+    return edge_base<K, F>(t) + edge_step<K, F>(m);
 }
 
 // A thread's 16 residues in the edge layout from / to the tile at p: groups of four as one
@@ -163,9 +167,9 @@ struct PassTw {
 // Twiddles of the pass at bit 0, stage b, into w[0 .. 2^(3-b)): the lane-major copy (`lt`)
 // for four stages, else the table itself, whose lookups by neighbouring lanes are
 // neighbours in the edge layout; pairs as one 32-byte load.
-template <int K>
+template <int K, TileForm F>
 __device__ __forceinline__ void edge_tw(double2* w, int b, int t, int hi, int logP, const FCtx& c) {
-    constexpr int NST = EdgePass<K>::NST;
+    constexpr int NST = EdgePass<K, F>::NST;
     if constexpr (NST == 4) {
         // one twiddle per thread and slot: the lane-major copy keeps the warp's loads contiguous
         const int g = (hi << (K - 4)) + t;
@@ -175,7 +179,7 @@ __device__ __forceinline__ void edge_tw(double2* w, int b, int t, int hi, int lo
         const double2* T = c.tw + (1 << (logP - 1 - b)) + (hi << (K - b - 1));
 #pragma unroll
         for (int h = 0; h < (1 << (3 - b)); ++h) {
-            const double2* p = T + (edge_base<K>(t) >> (b + 1)) + (edge_step<K>(h << (b + 1)) >> (b + 1));
+            const double2* p = T + (edge_base<K, F>(t) >> (b + 1)) + (edge_step<K, F>(h << (b + 1)) >> (b + 1));
             if (b < NST - 1) {  // slots h and h + 1 are neighbours
                 if (h & 1) continue;
                 asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
@@ -191,16 +195,16 @@ __device__ __forceinline__ void edge_tw(double2* w, int b, int t, int hi, int lo
 // Whether a tile's exchange and forward twiddle addresses are left to the compiler: see fput_at.
 template <int K, TileForm F>
 __host__ __device__ constexpr bool whole_addresses() {
-    return EdgePass<K>::NST == 4 && F == kStraight;
+    return EdgePass<K, F>::NST == 4 && F == kWhole;
 }
 
-template <int K, int LO, int BHI, int BLO, TileForm F = kStraight>
+template <int K, int LO, int BHI, int BLO, TileForm F = kWhole>
 __device__ __forceinline__ void f_fwd_tw(PassTw<LO, BHI, BLO>& T, int t, int hi, int logP, const FCtx& c) {
 #pragma unroll
     for (int b = BHI; b >= BLO; --b) {
         const int bb = b - LO;
         if constexpr (LO == 0) {
-            edge_tw<K>(&T.w[PassTw<LO, BHI, BLO>::offset(b)], b, t, hi, logP, c);
+            edge_tw<K, F>(&T.w[PassTw<LO, BHI, BLO>::offset(b)], b, t, hi, logP, c);
         } else if constexpr (LO == 2 && K >= 6) {
             // four threads per 64-residue group: a warp's loads are 8 consecutive pairs
             const int g = (hi << (K - 6)) + (t >> 2);
@@ -250,14 +254,14 @@ __device__ __forceinline__ void f_fwd_bits(double (&x)[16], const PassTw<LO, BHI
 
 // Inverse stages at bits BLO..BHI of the field at LO.  FINAL: the global last bit folds
 // P^-1 (constants pinv and ilast, centred with their fl(./q) companions).
-template <int K, int LO, int BLO, int BHI, bool FINAL>
+template <int K, int LO, int BLO, int BHI, bool FINAL, TileForm F>
 __device__ __forceinline__ void f_inv_tw(PassTw<LO, BLO, BHI>& T, int t, int hi, int logP, const FCtx& c) {
 #pragma unroll
     for (int b = BLO; b <= BHI; ++b) {
         if (FINAL && b == BHI) break;  // the last stage uses the P^-1 constants
         const int bb = b - LO;
         if constexpr (LO == 0) {
-            edge_tw<K>(&T.w[PassTw<LO, BLO, BHI>::offset(b)], b, t, hi, logP, c);
+            edge_tw<K, F>(&T.w[PassTw<LO, BLO, BHI>::offset(b)], b, t, hi, logP, c);
         } else if constexpr (LO == 2 && K >= 6) {
             const int g = (hi << (K - 6)) + (t >> 2);
 #pragma unroll
@@ -304,44 +308,44 @@ __device__ __forceinline__ void f_inv_bits(double (&x)[16], const PassTw<LO, BLO
 }
 
 // Exchange reads and writes in the layout of the pass at LO (the edge layout at bit 0).
-template <int K, int LO>
+template <int K, int LO, TileForm F>
 __device__ __forceinline__ int slot_base(int t) {
-    return pad(LO == 0 ? edge_base<K>(t) : own_base<LO>(t));
+    return pad(LO == 0 ? edge_base<K, F>(t) : own_base<LO>(t));
 }
-template <int K, int LO>
+template <int K, int LO, TileForm F>
 __host__ __device__ __forceinline__ constexpr int slot_step(int m) {
-    return pad(LO == 0 ? edge_step<K>(m) : own_step<LO>(m));
+    return pad(LO == 0 ? edge_step<K, F>(m) : own_step<LO>(m));
 }
 
 // Tiles whose passes all have four stages (2^8, 2^12) leave these addresses, and the forward
-// twiddles', to the compiler where a kernel's tile code stands alone: with the split form their
+// twiddles', to the compiler where one transform is all of a kernel: with the split form their
 // forward launches ran 6% longer (2400 rows of 2^12: 65.6 us split, 59.3 so; 9600 rows 212),
-// the other tiles' shorter.  Kernels that walk tiles in a loop (kLooped) split them all the
-// same: whole addresses spill there (bytes a thread, whole and split: the work list's forward
+// the other tiles' shorter.  Ring products split them all the same (chain_form), and so do the
+// kernels that walk tiles in a loop: whole addresses spill there (bytes a thread, whole and split: the work list's forward
 // kernel 692 and 268, 2^12 tiles in persistent grids 464 and 0, in the dataflow kernel 292 and
 // 16; 2400 rows of 2^12 forward on one CTA an SM 145 us and 102).
-template <int K, int LO, TileForm F = kStraight>
+template <int K, int LO, TileForm F = kWhole>
 __device__ __forceinline__ void fput_at(double* sm, const double (&x)[16], int t) {
     if constexpr (whole_addresses<K, F>()) {
 #pragma unroll
         for (int m = 0; m < 16; ++m) sm[pad(own<LO>(t, m))] = x[m];
         return;
     }
-    double* p = sm + slot_base<K, LO>(t);
+    double* p = sm + slot_base<K, LO, F>(t);
 #pragma unroll
-    for (int m = 0; m < 16; ++m) p[slot_step<K, LO>(m)] = x[m];
+    for (int m = 0; m < 16; ++m) p[slot_step<K, LO, F>(m)] = x[m];
 }
 
-template <int K, int LO, TileForm F = kStraight>
+template <int K, int LO, TileForm F = kWhole>
 __device__ __forceinline__ void fget_at(double (&x)[16], const double* sm, int t) {
     if constexpr (whole_addresses<K, F>()) {
 #pragma unroll
         for (int m = 0; m < 16; ++m) x[m] = sm[pad(own<LO>(t, m))];
         return;
     }
-    const double* p = sm + slot_base<K, LO>(t);
+    const double* p = sm + slot_base<K, LO, F>(t);
 #pragma unroll
-    for (int m = 0; m < 16; ++m) x[m] = p[slot_step<K, LO>(m)];
+    for (int m = 0; m < 16; ++m) x[m] = p[slot_step<K, LO, F>(m)];
 }
 
 struct Tile {
@@ -450,7 +454,7 @@ __device__ __forceinline__ FCtx fwd_ctx(const PrimeInfo& pi) {
 // The forward passes of one tile whose 16 residues per thread are in x (x[m] at index
 // own<K - 4>(t, m), |x| <= q), the first pass's twiddles in tw1.  On return x[m] is at
 // index edge<K>(t, m) (|x| < 2^51, not reduced).
-template <int K, bool GROUP, TileForm F = kStraight>
+template <int K, bool GROUP, TileForm F = kWhole>
 __device__ __forceinline__ void tile_fwd_passes(const FCtx& c, int logP, int hi, double* sm, int t, double (&x)[16],
                                                 const PassTw<K - 4, K - 1, K - 4>& tw1, int grp) {
     constexpr int L1 = K - 4;
@@ -491,7 +495,7 @@ __device__ __forceinline__ void tile_fwd_passes(const FCtx& c, int logP, int hi,
 // when `store` is set (a thread whose tile only pads out a group computes without
 // storing).  GROUP, grp: the tile's threads synchronise at named barrier 1 + grp
 // (tile_sync).
-template <int K, bool IN_D, bool STAGED, bool GROUP = false, TileForm F = kStraight>
+template <int K, bool IN_D, bool STAGED, bool GROUP = false, TileForm F = kWhole>
 __device__ __forceinline__ void tile_fwd_regs(const Tile& r, int logP, bool red, double* sm, int t, double (&x)[16],
                                               int grp = 0) {
     const FCtx c = fwd_ctx(*r.pi);
@@ -514,7 +518,7 @@ __device__ __forceinline__ void tile_fwd_regs(const Tile& r, int logP, bool red,
     tile_fwd_passes<K, GROUP, F>(c, logP, hi, sm, t, x, tw1, grp);
 }
 
-template <int K, bool IN_D, bool STAGED, bool GROUP = false, TileForm F = kStraight>
+template <int K, bool IN_D, bool STAGED, bool GROUP = false, TileForm F = kWhole>
 __device__ __forceinline__ void tile_fwd_one(const Tile& r, const RowSet& rows, double* sm, int t, bool store,
                                              int grp = 0) {
     double x[16];
@@ -522,29 +526,30 @@ __device__ __forceinline__ void tile_fwd_one(const Tile& r, const RowSet& rows, 
     if (store) store_edge_canonical<K>(r.dst, x, t, r.pi->qd, r.pi->qinv, r.pi->q);
 }
 
-// Passes of the inverse from bit LO up, four stages each, after the pass below left its
-// residues in layout PREV.
-template <int K, int PREV, int LO, bool FINAL, bool GROUP, TileForm F>
+// Passes of the inverse from bit B up, four stages each (the last those that are left), after
+// the pass below left its residues in layout PREV.
+template <int K, int PREV, int B, bool FINAL, bool GROUP, TileForm F>
 __device__ __forceinline__ void tile_inv_passes(const PrimeInfo& pi, const FCtx& c, int logP, int hi, double* sm, int t,
                                                 double (&x)[16], int grp) {
-    constexpr bool last = LO + 4 == K;
-    PassTw<LO, LO, LO + 3> tw;
-    f_inv_tw<K, LO, LO, LO + 3, FINAL && last>(tw, t, hi, logP, c);
+    constexpr int LO = B < K - 4 ? B : K - 4, TOP = B + 3 < K - 1 ? B + 3 : K - 1;
+    constexpr bool last = TOP == K - 1;
+    PassTw<LO, B, TOP> tw;
+    f_inv_tw<K, LO, B, TOP, FINAL && last, F>(tw, t, hi, logP, c);
     if (PREV > 0) tile_sync<K, GROUP>(grp);  // the previous exchange is read
     fput_at<K, PREV, F>(sm, x, t);
     tile_sync<K, GROUP>(grp);
     fget_at<K, LO, F>(x, sm, t);
-    f_inv_bits<K, LO, LO, LO + 3, FINAL && last>(x, tw, c, pi);
-    if constexpr (!last) tile_inv_passes<K, LO, LO + 4, FINAL, GROUP, F>(pi, c, logP, hi, sm, t, x, grp);
+    f_inv_bits<K, LO, B, TOP, FINAL && last>(x, tw, c, pi);
+    if constexpr (!last) tile_inv_passes<K, LO, TOP + 1, FINAL, GROUP, F>(pi, c, logP, hi, sm, t, x, grp);
 }
 
 // Inverse passes of the low K bits of one tile whose 16 residues per thread t are in x
 // (x[m] at index edge<K>(t, m), |x| < q; the forward passes leave this layout).  FINAL
 // (K == logP): P^-1 folded in.  On return x[m] is at index own<K - 4>(t, m) of the tile.
-template <int K, bool FINAL, bool GROUP = false, TileForm F = kStraight>
+template <int K, bool FINAL, bool GROUP = false, TileForm F = kWhole>
 __device__ __forceinline__ void tile_inv_regs(const PrimeInfo& pi, int logP, int hi, double* sm, int t,
                                               double (&x)[16], int grp = 0) {
-    constexpr int NST = EdgePass<K>::NST;
+    constexpr int NST = EdgePass<K, F>::NST;
     FCtx c;
     c.q = pi.qd;
     c.qinv = pi.qinv;
@@ -552,7 +557,7 @@ __device__ __forceinline__ void tile_inv_regs(const PrimeInfo& pi, int logP, int
     c.lt = reinterpret_cast<const double2*>(pi.inv_lane);
     c.mt = reinterpret_cast<const double2*>(pi.inv_mid);
     PassTw<0, 0, NST - 1> tw1;
-    f_inv_tw<K, 0, 0, NST - 1, false>(tw1, t, hi, logP, c);
+    f_inv_tw<K, 0, 0, NST - 1, false, F>(tw1, t, hi, logP, c);
     f_inv_bits<K, 0, 0, NST - 1, false>(x, tw1, c, pi);
     tile_inv_passes<K, 0, NST, FINAL, GROUP, F>(pi, c, logP, hi, sm, t, x, grp);
 }
@@ -560,7 +565,7 @@ __device__ __forceinline__ void tile_inv_regs(const PrimeInfo& pi, int logP, int
 // Inverse transform of the low K bits of tile r.  FINAL (K == logP): P^-1 folded in,
 // canonical output; otherwise centred doubles for the column pass.  STAGED and store as
 // for tile_fwd_one.
-template <int K, bool FINAL, bool STAGED, bool GROUP = false, TileForm F = kStraight>
+template <int K, bool FINAL, bool STAGED, bool GROUP = false, TileForm F = kWhole>
 __device__ __forceinline__ void tile_inv_one(const Tile& r, const RowSet& rows, double* sm, int t, bool store,
                                              int grp = 0) {
     const PrimeInfo& pi = *r.pi;

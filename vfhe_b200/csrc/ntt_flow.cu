@@ -137,8 +137,8 @@ __global__ void __launch_bounds__(TileThreads<K>::value, TileMinBlocks<K>::value
                 const RowSet& rs = INV ? a : b;
                 const Tile r = locate<false>(rs, primes, K, (row << K1) + item * G + lt, 1 << K1);
                 if (s) tile_sync<K, GROUP>(lt);  // the previous tile's exchanges are over
-                if (INV) tile_inv_one<K, false, false, GROUP, kLooped>(r, rs, sm, t, true, lt);
-                else tile_fwd_one<K, true, false, GROUP, kLooped>(r, rs, sm, t, true, lt);
+                if (INV) tile_inv_one<K, false, false, GROUP, kSplit>(r, rs, sm, t, true, lt);
+                else tile_fwd_one<K, true, false, GROUP, kSplit>(r, rs, sm, t, true, lt);
             }
         }
         __syncthreads();  // the ticket's stores are issued and every thread has read s_item

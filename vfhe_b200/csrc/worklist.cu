@@ -264,8 +264,8 @@ __device__ __forceinline__ void wl_tiles(const RowSet& rows, double* fsm) {
         const long long tile = grp * TPC + lt;
         const bool valid = tile < ntiles;
         const Tile r = locate<true>(rows, nullptr, K, valid ? tile : ntiles - 1, tiles_per_row);
-        if constexpr (INV) tile_inv_one<K, !TWO, false, false, kLooped>(r, rows, sm, t, valid);
-        else tile_fwd_one<K, TWO, false, false, kLooped>(r, rows, sm, t, valid);
+        if constexpr (INV) tile_inv_one<K, !TWO, false, false, kSplit>(r, rows, sm, t, valid);
+        else tile_fwd_one<K, TWO, false, false, kSplit>(r, rows, sm, t, valid);
         __syncthreads();  // the next step reuses the exchange buffers
     }
 }
