@@ -154,11 +154,17 @@ __global__ void __launch_bounds__(TileThreads<K>::value, TileMinBlocks<K>::value
 // barriers here): an SM takes the next columns as each warp pair ends instead of as four
 // or eight warps do, which counts where a launch is two or three waves.  319 rows of 2^14
 // points, both passes: 43.05 us with 256 threads, 42.4 with 128, 42.0 with 64; 75 rows of 2^16
-// by 24 digits 1421 -> 1413; large launches equal.
-constexpr int COLT = 64;
+// by 24 digits 1421 -> 1413; large launches equal.  A radix-2 thread has two residues, and in
+// CTAs of 64 the CTA rate bounds it (1536 rows of 2^13 by 2^12 tiles, forward and inverse:
+// 123.9 and 124.8 us with 64, 111.2 and 111.4 with 128, 111.7 and 112.0 with 256).
+template <int K1>
+struct ColThreads {
+    static constexpr int value = K1 == 1 ? 128 : 64;
+};
+
 template <int K1, bool INV>
-__global__ void __launch_bounds__(COLT, (K1 >= 5 ? 512 : 1024) / COLT) k_col_f(const __grid_constant__ RowSet rows,
-                                               const PrimeInfo* __restrict__ primes, long long ncols, int KT) {
+__global__ void __launch_bounds__(ColThreads<K1>::value, (K1 >= 5 ? 512 : 1024) / ColThreads<K1>::value)
+    k_col_f(const __grid_constant__ RowSet rows, const PrimeInfo* __restrict__ primes, long long ncols, int KT) {
     const long long gc = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (gc >= ncols) return;  // no barriers in this kernel
     col_one<K1, INV>(rows, primes, gc, KT);
@@ -387,9 +393,10 @@ int tile_launch(const RowSet& rows, const PrimeInfo* d_primes, int mode, int til
 template <int K1>
 int col_launch(const RowSet& rows, const PrimeInfo* d_primes, bool inverse, int KT, cudaStream_t st) {
     const long long ncols = rowset_rows(rows) << KT;
-    const long long grid = (ncols + COLT - 1) / COLT;
-    if (inverse) k_col_f<K1, true><<<(unsigned)grid, COLT, 0, st>>>(rows, d_primes, ncols, KT);
-    else k_col_f<K1, false><<<(unsigned)grid, COLT, 0, st>>>(rows, d_primes, ncols, KT);
+    constexpr int T = ColThreads<K1>::value;
+    const long long grid = (ncols + T - 1) / T;
+    if (inverse) k_col_f<K1, true><<<(unsigned)grid, T, 0, st>>>(rows, d_primes, ncols, KT);
+    else k_col_f<K1, false><<<(unsigned)grid, T, 0, st>>>(rows, d_primes, ncols, KT);
     note_launch();
     return (int)cudaGetLastError();
 }
