@@ -183,6 +183,11 @@ constexpr size_t kTileSmemMax = 200 * 1024;
 // the low K bits are then the usual register-blocked tile passes, fed from shared
 // memory.  The row crosses HBM once in and once out, instead of twice each way for
 // the column kernel + tile kernel pair, and it is one launch.
+//
+// Tile forms: split addresses (192 rows of 2^13 on 2^12 tiles, forward: 19.8 us whole, 17.0
+// split), and 16 consecutive residues a thread where a 2^13 tile starts the inverse (192 rows
+// of 2^16: 197 us with the edge layout, 190 so; forward 185 and 200, and smaller tiles are
+// longer so in both directions).
 namespace cgx = cooperative_groups;
 
 template <int K, int K1, bool TABLE>
@@ -241,11 +246,11 @@ __global__ void __launch_bounds__(TileThreads<K>::value) k_fused_fwd_f(const __g
     double x[16];
     constexpr int L1 = K - 4;
     PassTw<L1, K - 1, L1> tw1;
-    f_fwd_tw<K, L1, K - 1, L1>(tw1, t, hi, logP, c);
+    f_fwd_tw<K, L1, K - 1, L1, kSplit>(tw1, t, hi, logP, c);
 #pragma unroll
     for (int m = 0; m < 16; ++m) x[m] = fsm[own<L1>(t, m)];
     __syncthreads();  // every value is in registers before the exchanges reuse the buffer
-    tile_fwd_passes<K, false>(c, logP, hi, fsm, t, x, tw1, 0);
+    tile_fwd_passes<K, false, kSplit>(c, logP, hi, fsm, t, x, tw1, 0);
     store_edge_canonical<K>(r.dst, x, t, c.q, c.qinv, pi.q);
 }
 
@@ -269,8 +274,9 @@ __global__ void __launch_bounds__(TileThreads<K>::value) k_fused_inv_f(const __g
     const int logP = rows.logP, hi = rank;
     // phase 1: inverse tile passes over the low K bits of this block
     double x[16];
-    load_edge_u64<K>(x, r.src, t);
-    tile_inv_regs<K, false>(pi, logP, hi, fsm, t, x);
+    constexpr TileForm F = K == 13 ? kLinear : kSplit;
+    load_edge_u64<K, F>(x, r.src, t);
+    tile_inv_regs<K, false, false, F>(pi, logP, hi, fsm, t, x);
     constexpr int LAST = K - 4;
     __syncthreads();  // the exchanges are over: the block goes back in natural order
 #pragma unroll

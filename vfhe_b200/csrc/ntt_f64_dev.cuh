@@ -91,16 +91,16 @@ __device__ __forceinline__ int edge(int t, int m) {
 
 // A thread's 16 residues in the edge layout from / to the tile at p: groups of four as one
 // 32-byte access when the tile is 32-byte aligned, 16-byte accesses otherwise.
-template <int K>
+template <int K, TileForm F = kWhole>
 __device__ __forceinline__ void load_edge_u64(double (&x)[16], const uint64_t* p, int t) {
-    if (EdgePass<K>::NST >= 2 && (reinterpret_cast<uintptr_t>(p) & 31) == 0) {
+    if (EdgePass<K, F>::NST >= 2 && (reinterpret_cast<uintptr_t>(p) & 31) == 0) {
 #pragma unroll
         for (int m = 0; m < 16; m += 4) {
             uint64_t a, b, c, d;
             // ordered like an ordinary load: rows may be transformed in place
             asm volatile("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];"
                          : "=l"(a), "=l"(b), "=l"(c), "=l"(d)
-                         : "l"(p + edge<K>(t, m))
+                         : "l"(p + edge<K, F>(t, m))
                          : "memory");
             x[m] = f_from_u64(a);
             x[m + 1] = f_from_u64(b);
@@ -110,22 +110,22 @@ __device__ __forceinline__ void load_edge_u64(double (&x)[16], const uint64_t* p
     } else {
 #pragma unroll
         for (int m = 0; m < 16; m += 2) {
-            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p + edge<K>(t, m));
+            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p + edge<K, F>(t, m));
             x[m] = f_from_u64(v.x);
             x[m + 1] = f_from_u64(v.y);
         }
     }
 }
 
-template <int K>
+template <int K, TileForm F = kWhole>
 __device__ __forceinline__ void store_edge_canonical(uint64_t* p, const double (&x)[16], int t, double q, double qinv,
                                                      uint64_t qi) {
-    if (EdgePass<K>::NST >= 2 && (reinterpret_cast<uintptr_t>(p) & 31) == 0) {
+    if (EdgePass<K, F>::NST >= 2 && (reinterpret_cast<uintptr_t>(p) & 31) == 0) {
 #pragma unroll
         for (int m = 0; m < 16; m += 4) {
             const uint64_t a = f_to_canonical(x[m], q, qinv, qi), b = f_to_canonical(x[m + 1], q, qinv, qi);
             const uint64_t c = f_to_canonical(x[m + 2], q, qinv, qi), d = f_to_canonical(x[m + 3], q, qinv, qi);
-            asm volatile("st.global.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(p + edge<K>(t, m)), "l"(a), "l"(b), "l"(c),
+            asm volatile("st.global.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(p + edge<K, F>(t, m)), "l"(a), "l"(b), "l"(c),
                          "l"(d)
                          : "memory");
         }
@@ -135,7 +135,7 @@ __device__ __forceinline__ void store_edge_canonical(uint64_t* p, const double (
             ulonglong2 v;
             v.x = f_to_canonical(x[m], q, qinv, qi);
             v.y = f_to_canonical(x[m + 1], q, qinv, qi);
-            *reinterpret_cast<ulonglong2*>(p + edge<K>(t, m)) = v;
+            *reinterpret_cast<ulonglong2*>(p + edge<K, F>(t, m)) = v;
         }
     }
 }
@@ -523,7 +523,7 @@ __device__ __forceinline__ void tile_fwd_one(const Tile& r, const RowSet& rows, 
                                              int grp = 0) {
     double x[16];
     tile_fwd_regs<K, IN_D, STAGED, GROUP, F>(r, rows.logP, rows.reduce_input != 0, sm, t, x, grp);
-    if (store) store_edge_canonical<K>(r.dst, x, t, r.pi->qd, r.pi->qinv, r.pi->q);
+    if (store) store_edge_canonical<K, F>(r.dst, x, t, r.pi->qd, r.pi->qinv, r.pi->q);
 }
 
 // Passes of the inverse from bit B up, four stages each (the last those that are left), after
@@ -544,7 +544,7 @@ __device__ __forceinline__ void tile_inv_passes(const PrimeInfo& pi, const FCtx&
 }
 
 // Inverse passes of the low K bits of one tile whose 16 residues per thread t are in x
-// (x[m] at index edge<K>(t, m), |x| < q; the forward passes leave this layout).  FINAL
+// (x[m] at index edge<K, F>(t, m), |x| < q; the forward passes leave this layout).  FINAL
 // (K == logP): P^-1 folded in.  On return x[m] is at index own<K - 4>(t, m) of the tile.
 template <int K, bool FINAL, bool GROUP = false, TileForm F = kWhole>
 __device__ __forceinline__ void tile_inv_regs(const PrimeInfo& pi, int logP, int hi, double* sm, int t,
@@ -574,12 +574,12 @@ __device__ __forceinline__ void tile_inv_one(const Tile& r, const RowSet& rows, 
         const uint64_t* in = reinterpret_cast<const uint64_t*>(sm);
 #pragma unroll
         for (int m = 0; m < 16; m += 2) {
-            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(in + edge<K>(t, m));
+            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(in + edge<K, F>(t, m));
             x[m] = f_from_u64(v.x);
             x[m + 1] = f_from_u64(v.y);
         }
     } else {
-        load_edge_u64<K>(x, r.src, t);
+        load_edge_u64<K, F>(x, r.src, t);
     }
     if (STAGED) tile_sync<K, GROUP>(grp);  // every input is in registers before the exchanges reuse the buffer
     tile_inv_regs<K, FINAL, GROUP, F>(pi, rows.logP, r.hi, sm, t, x, grp);
