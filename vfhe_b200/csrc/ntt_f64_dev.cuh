@@ -211,6 +211,12 @@ __device__ __forceinline__ void f_fwd_tw(PassTw<LO, BHI, BLO>& T, int t, int hi,
 #pragma unroll
             for (int h = 0; h < (1 << (3 - bb)); ++h)
                 T.w[PassTw<LO, BHI, BLO>::offset(b) + h] = __ldg(&c.mt[lane_tw_index(g, bb, h)]);
+        } else if constexpr (whole_addresses<K, F>() && K == 8) {
+            // 32-bit indices: 24579 rows of 2^8 42.6 us with pointers, 42.0 so (2^12: 514 and 566)
+            const int base = (1 << (logP - 1 - b)) + (hi << (K - b - 1));
+#pragma unroll
+            for (int h = 0; h < (1 << (3 - bb)); ++h)
+                T.w[PassTw<LO, BHI, BLO>::offset(b) + h] = __ldg(&c.tw[base + (own<LO>(t, h << (bb + 1)) >> (b + 1))]);
         } else if constexpr (whole_addresses<K, F>()) {
             const double2* p = c.tw + (1 << (logP - 1 - b)) + (hi << (K - b - 1));
 #pragma unroll
