@@ -61,3 +61,15 @@ def test_rows_on_16_bytes(cuda, oracle_engine, log_p, schedule, in_place):
 def test_short_column_passes(cuda, oracle_engine, log_p, tile, rows):
     """Column passes of two and four points, in CTAs of 128 and 64 threads."""
     _check(cuda, oracle_engine, log_p, rows, (tile, 0, 0), 0, True)
+
+
+@pytest.mark.parametrize("log_p,tile", [(9, 9), (10, 10), (11, 11), (12, 12), (13, 11), (14, 13)])
+@pytest.mark.parametrize("side", [0, 1])
+def test_inverse_forms(cuda, oracle_engine, log_p, tile, side):
+    """Tile counts on both sides of the inverse kernels' rule: one CTA's threads an SM at 2^10
+    and 2^11, four tiles an SM at 2^12."""
+    import torch
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    tiles = {9: 8 * sms, 10: 4 * sms, 11: 2 * sms, 12: 4 * sms, 13: sms}[tile]
+    _check(cuda, oracle_engine, log_p, (tiles >> (log_p - tile)) + side, (tile, 1, 0), 0, False)

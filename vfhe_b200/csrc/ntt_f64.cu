@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(TileThreads<K>::value, TileMinBlocks<K>::value
 
 // Inverse transform of the low K bits.  FINAL (K == logP): P^-1 folded in, canonical
 // output; otherwise centred doubles are written for the column pass.
-template <int K, bool FINAL, bool PERSIST, bool TABLE>
+template <int K, bool FINAL, bool PERSIST, bool TABLE, TileForm F>
 __global__ void __launch_bounds__(TileThreads<K>::value, TileMinBlocks<K>::value) k_tile_inv_f(const __grid_constant__ RowSet rows,
                                                                      const PrimeInfo* __restrict__ primes,
                                                                      int tiles_per_cta, int tiles_per_row,
@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(TileThreads<K>::value, TileMinBlocks<K>::value
     }
     const long long tile = grp * tiles_per_cta + lt;
     const Tile r = locate<TABLE>(rows, primes, K, tile, tiles_per_row);
-    tile_inv_one<K, FINAL, PERSIST, false, PERSIST ? kSplit : kWhole>(r, rows, sm, t, true);
+    tile_inv_one<K, FINAL, PERSIST, false, F>(r, rows, sm, t, true);
     if (!PERSIST) break;
     __syncthreads();  // the next trip rewrites shared memory
     }
@@ -340,6 +340,40 @@ int set_smem(KernelT kern, size_t bytes) {
     return e;
 }
 
+// Form of an inverse launch of `tiles` tiles.  The coalesced edge pass pays where the L1 pipe is
+// busy; with less than one CTA's warps on an SM the launch is one tile's latency, which 16
+// consecutive residues a thread keep shorter (one wide load instead of several narrow ones, a
+// four-stage first pass).  us, edge and linear:
+//   2^9    always linear: 4092 rows 13.3 and 11.6, 24579 rows 55.0 and 54.6
+//   2^10   60 rows 4.40 and 4.25, 384 rows 5.22 and 5.02, 768 rows 6.54 and 6.57, 8187 rows 36.8 and 38.9
+//   2^11   before a column pass, 72 tiles 8.30 and 7.99, 192 tiles 8.74 and 8.44, 396 tiles 12.25 and 12.54
+//   2^13   before a column pass, 384 rows of 2^14 74.7 and 73.0; alone, 768 rows 54.8 and 55.8
+// 2^12 tiles have the same layout either way and split their addresses past four tiles an SM
+// (whole and split: 60 rows 6.11 and 6.28, 384 rows 12.2 and 12.3, 1536 rows 38.3 and 37.3,
+// 24579 rows 569 and 555).
+template <int K, bool FINAL>
+TileForm inverse_form(long long tiles) {
+    const long long threads = tiles << (K - 4), sms = sm_count();
+    if (K == 9) return kLinear;
+    if (K == 10 || K == 11) return threads <= 256 * sms ? kLinear : kWhole;
+    if (K == 12) return threads > 1024 * sms ? kSplit : kWhole;
+    return K == 13 && !FINAL ? kLinear : kWhole;
+}
+// The forms inverse_form can return for tiles of 2^K points.
+template <int K, bool FINAL, TileForm F>
+constexpr bool inverse_takes() {
+    if (K == 9) return F == kLinear;
+    if (K == 10 || K == 11) return F != kSplit;
+    if (K == 12) return F != kLinear;
+    return F == (K == 13 && !FINAL ? kLinear : kWhole);
+}
+// Persistent grids: linear at 2^9 (768 rows, two CTAs an SM, 9.3 us edge, 8.9 linear), split
+// addresses elsewhere.
+template <int K>
+constexpr TileForm inverse_persist_form() {
+    return K == 9 ? kLinear : kSplit;
+}
+
 // mode: 0 forward (canonical in), 1 forward (doubles in), 2 inverse final, 3 inverse to doubles
 template <int K>
 int tile_launch(const RowSet& rows, const PrimeInfo* d_primes, int mode, int tiles_per_row, const NttSchedule& sc,
@@ -371,7 +405,13 @@ int tile_launch(const RowSet& rows, const PrimeInfo* d_primes, int mode, int til
         e = set_smem(KERN, smem);                                                                         \
         if (!e) KERN<<<(unsigned)grid, threads, smem, st>>>(rows, d_primes, tiles_per_cta, tiles_per_row, ngroups); \
     } while (0)
+#define VC_TILE_INV(FINAL, TABLE, F)                                                        \
+    do {                                                                                    \
+        if constexpr (inverse_takes<K, FINAL, F>())                                         \
+            if (form == F) VC_TILE_LAUNCH((k_tile_inv_f<K, FINAL, false, TABLE, F>));       \
+    } while (0)
     const bool table = rows.table != nullptr;
+    const TileForm form = mode == 2 ? inverse_form<K, true>(ntiles) : inverse_form<K, false>(ntiles);
     switch (mode * 4 + (persist ? 2 : 0) + (table ? 1 : 0)) {
         case 0: VC_TILE_LAUNCH((k_tile_fwd_f<K, false, false, false>)); break;
         case 1: VC_TILE_LAUNCH((k_tile_fwd_f<K, false, false, true>)); break;
@@ -381,15 +421,16 @@ int tile_launch(const RowSet& rows, const PrimeInfo* d_primes, int mode, int til
         case 5: VC_TILE_LAUNCH((k_tile_fwd_f<K, true, false, true>)); break;
         case 6: VC_TILE_LAUNCH((k_tile_fwd_f<K, true, true, false>)); break;
         case 7: VC_TILE_LAUNCH((k_tile_fwd_f<K, true, true, true>)); break;
-        case 8: VC_TILE_LAUNCH((k_tile_inv_f<K, true, false, false>)); break;
-        case 9: VC_TILE_LAUNCH((k_tile_inv_f<K, true, false, true>)); break;
-        case 10: VC_TILE_LAUNCH((k_tile_inv_f<K, true, true, false>)); break;
-        case 11: VC_TILE_LAUNCH((k_tile_inv_f<K, true, true, true>)); break;
-        case 12: VC_TILE_LAUNCH((k_tile_inv_f<K, false, false, false>)); break;
-        case 13: VC_TILE_LAUNCH((k_tile_inv_f<K, false, false, true>)); break;
-        case 14: VC_TILE_LAUNCH((k_tile_inv_f<K, false, true, false>)); break;
-        default: VC_TILE_LAUNCH((k_tile_inv_f<K, false, true, true>)); break;
+        case 8: VC_TILE_INV(true, false, kWhole); VC_TILE_INV(true, false, kSplit); VC_TILE_INV(true, false, kLinear); break;
+        case 9: VC_TILE_INV(true, true, kWhole); VC_TILE_INV(true, true, kSplit); VC_TILE_INV(true, true, kLinear); break;
+        case 10: VC_TILE_LAUNCH((k_tile_inv_f<K, true, true, false, inverse_persist_form<K>()>)); break;
+        case 11: VC_TILE_LAUNCH((k_tile_inv_f<K, true, true, true, inverse_persist_form<K>()>)); break;
+        case 12: VC_TILE_INV(false, false, kWhole); VC_TILE_INV(false, false, kSplit); VC_TILE_INV(false, false, kLinear); break;
+        case 13: VC_TILE_INV(false, true, kWhole); VC_TILE_INV(false, true, kSplit); VC_TILE_INV(false, true, kLinear); break;
+        case 14: VC_TILE_LAUNCH((k_tile_inv_f<K, false, true, false, inverse_persist_form<K>()>)); break;
+        default: VC_TILE_LAUNCH((k_tile_inv_f<K, false, true, true, inverse_persist_form<K>()>)); break;
     }
+#undef VC_TILE_INV
 #undef VC_TILE_LAUNCH
     if (e) return e;
     note_launch();
@@ -485,12 +526,27 @@ int col_dispatch(int K1, const RowSet& rows, const PrimeInfo* d, bool inverse, i
 
 NttSchedule g_sched[kSchedMaxLogP + 1][kSchedRowBuckets];
 
-template <int K, bool P, bool T>
-int prepare_kp() {
-    int e = set_smem(k_tile_fwd_f<K, false, P, T>, kTileSmemMax);
-    if (!e) e = set_smem(k_tile_fwd_f<K, true, P, T>, kTileSmemMax);
-    if (!e) e = set_smem(k_tile_inv_f<K, true, P, T>, kTileSmemMax);
-    if (!e) e = set_smem(k_tile_inv_f<K, false, P, T>, kTileSmemMax);
+template <int K, bool FINAL, bool T, TileForm F>
+int prepare_inv() {
+    if constexpr (inverse_takes<K, FINAL, F>()) return set_smem(k_tile_inv_f<K, FINAL, false, T, F>, kTileSmemMax);
+    return 0;
+}
+
+template <int K, bool T>
+int prepare_kt() {
+    constexpr TileForm P = inverse_persist_form<K>();
+    int e = set_smem(k_tile_fwd_f<K, false, false, T>, kTileSmemMax);
+    if (!e) e = set_smem(k_tile_fwd_f<K, true, false, T>, kTileSmemMax);
+    if (!e) e = set_smem(k_tile_fwd_f<K, false, true, T>, kTileSmemMax);
+    if (!e) e = set_smem(k_tile_fwd_f<K, true, true, T>, kTileSmemMax);
+    if (!e) e = set_smem(k_tile_inv_f<K, true, true, T, P>, kTileSmemMax);
+    if (!e) e = set_smem(k_tile_inv_f<K, false, true, T, P>, kTileSmemMax);
+    if (!e) e = prepare_inv<K, true, T, kWhole>();
+    if (!e) e = prepare_inv<K, true, T, kSplit>();
+    if (!e) e = prepare_inv<K, true, T, kLinear>();
+    if (!e) e = prepare_inv<K, false, T, kWhole>();
+    if (!e) e = prepare_inv<K, false, T, kSplit>();
+    if (!e) e = prepare_inv<K, false, T, kLinear>();
     return e;
 }
 
@@ -505,10 +561,8 @@ int prepare_fused() {
 
 template <int K>
 int prepare_k() {
-    int e = prepare_kp<K, false, false>();
-    if (!e) e = prepare_kp<K, false, true>();
-    if (!e) e = prepare_kp<K, true, false>();
-    if (!e) e = prepare_kp<K, true, true>();
+    int e = prepare_kt<K, false>();
+    if (!e) e = prepare_kt<K, true>();
     if constexpr (K >= 11) {
         if (!e) e = prepare_fused<K, 1>();
         if (!e) e = prepare_fused<K, 2>();
