@@ -348,12 +348,13 @@ int set_smem(KernelT kern, size_t bytes) {
 //   2^10   60 rows 4.40 and 4.25, 384 rows 5.22 and 5.02, 768 rows 6.54 and 6.57, 8187 rows 36.8 and 38.9
 //   2^11   before a column pass, 72 tiles 8.30 and 7.99, 192 tiles 8.74 and 8.44, 396 tiles 12.25 and 12.54
 //   2^13   before a column pass, 384 rows of 2^14 74.7 and 73.0; alone, 768 rows 54.8 and 55.8
-// 2^12 tiles have the same layout either way and split their addresses past four tiles an SM
-// (whole and split: 60 rows 6.11 and 6.28, 384 rows 12.2 and 12.3, 1536 rows 38.3 and 37.3,
-// 24579 rows 569 and 555).
+// 2^8 and 2^12 tiles have the same layout either way.  2^8 split their addresses (24579 rows
+// 42.8 us whole, 42.4 split), 2^12 past four tiles an SM (whole and split: 60 rows 6.11 and
+// 6.28, 384 rows 12.2 and 12.3, 1536 rows 38.3 and 37.3, 24579 rows 569 and 555).
 template <int K, bool FINAL>
 TileForm inverse_form(long long tiles) {
     const long long threads = tiles << (K - 4), sms = sm_count();
+    if (K == 8) return kSplit;
     if (K == 9) return kLinear;
     if (K == 10 || K == 11) return threads <= 256 * sms ? kLinear : kWhole;
     if (K == 12) return threads > 1024 * sms ? kSplit : kWhole;
@@ -362,6 +363,7 @@ TileForm inverse_form(long long tiles) {
 // The forms inverse_form can return for tiles of 2^K points.
 template <int K, bool FINAL, TileForm F>
 constexpr bool inverse_takes() {
+    if (K == 8) return F == kSplit;
     if (K == 9) return F == kLinear;
     if (K == 10 || K == 11) return F != kSplit;
     if (K == 12) return F != kLinear;
