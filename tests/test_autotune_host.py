@@ -66,3 +66,25 @@ def test_dataflow_candidates_cover_the_two_pass_sizes():
     assert flows[16] == [12, 13] and flows[17] == [13]
     assert all(not flows[lp] for lp in range(8, 12))
 
+
+def test_a_class_is_timed_over_its_range():
+    from vfhe_b200.autotune import BUCKETS, row_counts
+
+    for b in BUCKETS:
+        counts = row_counts(b)
+        assert len(counts) == 3 and all(c >> b == 1 and c % 3 == 0 for c in counts)
+        assert any(c % 2 for c in counts) and any(c % (1 << (b - 1)) == 0 for c in counts)
+        assert counts[-1] > 1.7 * (1 << b)
+
+
+def test_choice_holds_over_every_row_count():
+    """A schedule that is fast at the class's power of two and twice as slow at an odd count
+    loses to one that is a little faster everywhere; less than 1% keeps the built-in one."""
+    from vfhe_b200.autotune import choose
+
+    default, peaky, steady = (9, 0, 0), (9, 4, 2), (9, 2, 0)
+    timed = [{default: 1.0, peaky: 0.8, steady: 0.95}, {default: 1.3, peaky: 2.6, steady: 1.2},
+             {default: 1.9, peaky: 1.7, steady: 1.8}]
+    assert choose(timed, default)[0] == steady
+    assert choose([{default: 1.0, steady: 0.995}], default) == (default, 1.0, 1.0)
+    assert choose([{peaky: 2.0, steady: 1.0}], default) == (steady, 1.0, None)
