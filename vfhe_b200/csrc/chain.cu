@@ -210,13 +210,15 @@ constexpr size_t chain_smem() {
 }
 
 // Most rows the 8-residue kernel takes: any number at (9, 4), one row an SM where a row is
-// 512 threads in split blocks (two of the 16-residue kernel's CTAs share an SM beyond that),
-// none elsewhere.
+// 512 threads in split blocks (two of the 16-residue kernel's CTAs share an SM beyond that).
+// Other shapes have no such kernel.
+template <int K, int S>
+constexpr bool chain8_built() {
+    return S > 1 && ((K == 9 && S == 4) || S << (K - 3) == 512);
+}
 template <int K, int S>
 long long chain8_rows() {
-    if constexpr (K == 9 && S == 4) return 0x7fffffffLL;
-    else if constexpr (S > 1 && S << (K - 3) == 512) return sm_count();
-    else return 0;
+    return K == 9 && S == 4 ? 0x7fffffffLL : sm_count();
 }
 
 template <int K, int S>
@@ -225,7 +227,7 @@ int chain_attr() {
     if (chain_smem<K, S>() > 48 * 1024)
         e = (int)cudaFuncSetAttribute(k_chain_f<K, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)chain_smem<K, S>());
-    if constexpr (S > 1 && S << (K - 3) <= 512) {
+    if constexpr (chain8_built<K, S>()) {
         if (!e && chain8_smem<K, S>() > 48 * 1024)
             e = (int)cudaFuncSetAttribute(k_chain8_f<K, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)chain8_smem<K, S>());
@@ -243,7 +245,7 @@ int chain_launch(uint64_t* out, const uint64_t* a, const uint64_t* b, long long 
     std::call_once(once, [] { attr_err = chain_attr<K, S>(); });
     if (attr_err) return attr_err;
     bool eight = false;
-    if constexpr (S > 1 && S << (K - 3) <= 512) {
+    if constexpr (chain8_built<K, S>()) {
         eight = rows <= chain8_rows<K, S>();
         if (eight) k_chain8_f<K, S><<<(unsigned)rows, S << (K - 3), chain8_smem<K, S>(), st>>>(out, a, b, cl, d, nl);
     }
