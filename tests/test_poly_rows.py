@@ -44,3 +44,31 @@ def test_rows_into_a_given_array(oracle_engine):
 @pytest.mark.gpu
 def test_rows_into_a_given_array_cuda(cuda):
     _given_arrays(cuda)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [[0, 1, 2], [0, 2], [2, 1, 0], [1, 2], [0, 1, 1, 2], [2], []])
+def test_read_rows_over_gaps_and_runs(cuda, rows):
+    """Runs of neighbouring rows go in one copy; any order, gaps and repeats give the same rows."""
+    p, want = _poly(cuda)
+    idx = [p.ring.prime_indices[k] for k in rows]
+    out = np.zeros((len(rows) + 1, N), dtype=np.uint64)
+    assert cuda.lib.vfhe_cuda_poly_read_rows(p.obj, cuda.ffi.from_buffer("uint64_t[]", out),
+                                             cuda.ffi.new("uint32_t[]", idx), len(idx)) == 0
+    assert np.array_equal(out[:-1], want[rows]) and not out[-1].any()
+
+
+@pytest.mark.gpu
+def test_read_rows_refusals(cuda):
+    p, _ = _poly(cuda)
+    lib, ffi = cuda.lib, cuda.ffi
+    out = np.zeros((2, N), dtype=np.uint64)
+    buf, one = ffi.from_buffer("uint64_t[]", out), ffi.new("uint32_t[]", [p.ring.prime_indices[0]])
+    outside = ffi.new("uint32_t[]", [p.ring.prime_indices[0], 63])
+    for args, what in (((p.obj, buf, outside, 2), "row outside"), ((p.obj, ffi.NULL, one, 1), "null"),
+                       ((p.obj, buf, ffi.NULL, 1), "null"), ((ffi.NULL, buf, one, 1), "")):
+        assert lib.vfhe_cuda_poly_read_rows(*args) != 0
+        assert what in ffi.string(lib.vfhe_cuda_last_error()).decode()
+        lib.vfhe_cuda_clear_error()
+    assert not out.any()
+    assert lib.vfhe_cuda_poly_read_rows(p.obj, ffi.NULL, ffi.NULL, 0) == 0  # nothing asked for
