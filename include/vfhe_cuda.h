@@ -543,7 +543,7 @@ int vfhe_cuda_worklist_phase_ms(void *wl, double *out6);
  *   One persistent launch: every CTA runs whole blind rotations with its accumulator
  *   in shared memory (wider CTAs for at most one ciphertext per SM).
  * keyswitch_batch: d_in [batch][N+1] -> d_out [batch][n+1] with d_ksk [N][levels][n+1]
- *   (base 2^base_log, signed digits); exact integer arithmetic.
+ *   (base 2^base_log, signed digits, base_log * levels <= 32); exact integer arithmetic.
  * external_product: d_out[b] = ExtProd(GGSW spectra d_ggsw_f, GLWE d_c[b] [2][N]) rounded
  *   to integers, and d_frac[b] = the largest distance of an unrounded coefficient to its
  *   integer (NULL to skip), for measuring the FFT error against exact products. */

@@ -488,7 +488,7 @@ int launch_cluster(int K, uint64_t* out_a, uint64_t* out_b, double* ext0, double
 // ext [B][2][L0 + 1][N].  Only the accumulator, the key and ext pass through L2; as four
 // launches (rotation difference, transforms, products, inverse) the digits and their spectra
 // did too.  Bound by the FP64 pipe's latency and rate: 1.1 M operations per LWE and step at
-// N = 1024, L0 = 2, 9 us of one SM.  1024 bootstraps at n = 630: 99 ms before, 73 ms.
+// N = 1024, L0 = 2, 9 us of one SM.  1024 bootstraps at n = 630: 99 ms before, 67.3 ms.
 template <int K, int L0>
 struct StepShape {
     static constexpr int N = 1 << K, NE = L0 + 1, ND = 2 * L0, TPT = 1 << (K - 4), THREADS = ND * TPT;

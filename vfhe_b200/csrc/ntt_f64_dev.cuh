@@ -459,7 +459,8 @@ __device__ __forceinline__ FCtx fwd_ctx(const PrimeInfo& pi) {
 
 // The forward passes of one tile whose 16 residues per thread are in x (x[m] at index
 // own<K - 4>(t, m), |x| <= q), the first pass's twiddles in tw1.  On return x[m] is at
-// index edge<K>(t, m) (|x| < 2^51, not reduced).
+// index edge<K, F>(t, m), not reduced: |x| < 4.3 q, past 2^52 for the largest primes (2^51 for
+// lazy ones), so f_reduce or f_to_canonical comes before any product.
 template <int K, bool GROUP, TileForm F = kWhole>
 __device__ __forceinline__ void tile_fwd_passes(const FCtx& c, int logP, int hi, double* sm, int t, double (&x)[16],
                                                 const PassTw<K - 4, K - 1, K - 4>& tw1, int grp) {
@@ -496,8 +497,8 @@ __device__ __forceinline__ void tile_fwd_passes(const FCtx& c, int logP, int hi,
 // Forward transform of the low K bits of tile r of a 2^logP-point row (16 residues per
 // thread t; the tile's padded exchange buffer at sm); red: reduce each input modulo the
 // row's prime on load.  STAGED: the input was copied into sm by a bulk copy; otherwise
-// it is read from r.src.  tile_fwd_regs leaves the result in x (x[m] at index edge<K>(t, m)
-// of the tile, |x| < 2^51, not reduced); tile_fwd_one stores it canonically to r.dst
+// it is read from r.src.  tile_fwd_regs leaves the result in x (x[m] at index edge<K, F>(t, m)
+// of the tile, |x| < 4.3 q, to be reduced before any product); tile_fwd_one stores it canonically to r.dst
 // when `store` is set (a thread whose tile only pads out a group computes without
 // storing).  GROUP, grp: the tile's threads synchronise at named barrier 1 + grp
 // (tile_sync).

@@ -331,8 +331,9 @@ __device__ __forceinline__ void wl_downs(const WlGroupPlan& G) {
 //   PART 2: inverse tile passes | barrier | inverse column passes of two-pass pools +
 //           divisions of one-pass pools | barrier | divisions of two-pass pools
 // Resident CTAs per SM asked of the compiler: three for the transform phases (80
-// registers; the forward phase spills 388 bytes per thread, yet two CTAs per SM at 128
-// registers without spills measured 5% slower), two for the MACs.
+// registers; the forward phase spills 268 bytes per thread, yet two CTAs per SM at 128
+// registers without spills are 4% slower: 64 jobs 3.24 against 3.11 ms, 512 jobs 26.0
+// against 25.0), two for the MACs.
 template <int PART>
 struct WlPartBlocks {
     static constexpr int value = PART == 1 ? 2 : 3;
