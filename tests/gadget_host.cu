@@ -15,6 +15,7 @@ static cudaError_t fake_last_error();
 #include <stdlib.h>
 
 #include <map>
+#include <utility>
 #include <string>
 
 namespace {
@@ -115,6 +116,11 @@ int main(int argc, char** argv) {
     if (g_case == "input_body_is_output_mask") in->b = out->a[0];
     if (g_case == "input_body_is_output_body") in->b = out->b;
     if (g_case == "input_mask_is_output_body") in->a[0] = out->b;
+    // rows that do not lie one after the other in the polynomial's block
+    auto swap_rows = [](RNS_Polynomial p) { std::swap(p->coeffs[0], p->coeffs[2]); };
+    if (g_case == "key_rows_moved") swap_rows(key[1]->b);
+    if (g_case == "output_rows_moved") swap_rows(out->a[0]);
+    if (g_case == "digit_rows_moved") swap_rows(in->a[0]);
     if (entry == "keyswitch") {
         void* comp[1] = {key};
         mlwe_RNSc_GHS_hybrid_keyswitch(out, in, comp, 0);

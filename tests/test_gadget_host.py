@@ -62,6 +62,13 @@ def test_shared_polynomials_go_digit_by_digit(calls, entry, case):
 
 
 @pytest.mark.parametrize("entry", ["keyswitch", "external_product"])
+@pytest.mark.parametrize("case", ["key_rows_moved", "output_rows_moved", "digit_rows_moved"])
+def test_rows_out_of_order_go_digit_by_digit(calls, entry, case):
+    """A polynomial's rows are where its row pointers say; the block's order is not assumed."""
+    assert calls(entry, case)["product"] >= 6
+
+
+@pytest.mark.parametrize("entry", ["keyswitch", "external_product"])
 def test_separate_polynomials_take_every_digit_at_once(calls, entry):
     got = calls(entry, "plain")
     assert got["alloc"] == got["free"] == (1 if entry == "keyswitch" else 2)

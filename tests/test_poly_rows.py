@@ -72,3 +72,15 @@ def test_read_rows_refusals(cuda):
         lib.vfhe_cuda_clear_error()
     assert not out.any()
     assert lib.vfhe_cuda_poly_read_rows(p.obj, ffi.NULL, ffi.NULL, 0) == 0  # nothing asked for
+
+
+@pytest.mark.gpu
+def test_read_rows_follow_the_row_pointers(cuda):
+    """Rows whose pointers the caller has exchanged are read where the pointers say."""
+    p, want = _poly(cuda)
+    c = cuda.ffi.cast("RNS_Polynomial", p.obj).coeffs
+    i, j = p.ring.prime_indices[0], p.ring.prime_indices[2]
+    c[i], c[j] = c[j], c[i]
+    got, seen = p.rows(), np.stack([p.row(k).copy() for k in p.ring.prime_indices])
+    c[i], c[j] = c[j], c[i]
+    assert np.array_equal(got, seen) and np.array_equal(got, want[[2, 1, 0]])

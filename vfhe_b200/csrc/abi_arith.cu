@@ -689,21 +689,21 @@ int vfhe_cuda_poly_read_rows(void* poly, uint64_t* h_out, const uint32_t* rows, 
     if (!valid_poly(poly, vc_where_)) return 1;
     Poly* p = as_poly(poly);
     const uint64_t N = p->pub.ntt->N;
-    if (count && (!h_out || !rows || !p->base)) {
+    if (count && (!h_out || !rows || !p->pub.coeffs)) {
         set_error(vc_where_, "null buffer, row list or rows");
         return 1;
     }
     for (uint32_t k = 0; k < count; ++k)
-        if (rows[k] >= p->pub.allocated_l) {
+        if (rows[k] >= p->pub.allocated_l || !p->pub.coeffs[rows[k]]) {
             set_error(vc_where_, "row outside the polynomial");
             return 1;
         }
-    // runs of neighbouring rows in one copy each
+    // runs of rows that lie one after the other in one copy each
     for (uint32_t k = 0; k < count;) {
+        const uint64_t* first = p->pub.coeffs[rows[k]];
         uint32_t n = 1;
-        while (k + n < count && rows[k + n] == rows[k] + n) ++n;
-        if (!VC_CHECK(cudaMemcpyAsync(h_out + (uint64_t)k * N, p->base + (uint64_t)rows[k] * N, n * N * sizeof(uint64_t),
-                                      cudaMemcpyDefault, stream())))
+        while (k + n < count && p->pub.coeffs[rows[k + n]] == first + n * N) ++n;
+        if (!VC_CHECK(cudaMemcpyAsync(h_out + (uint64_t)k * N, first, n * N * sizeof(uint64_t), cudaMemcpyDefault, stream())))
             return 1;
         k += n;
     }

@@ -256,14 +256,20 @@ int launch_gadget_mac(const GadgetMac& gm, const uint64_t* D, const PrimeInfo* p
 
 // Whether gadget_mac_all takes these operands: one pool, FP64 primes (the digits' own too: a
 // digit is read as a double before it is reduced), every key polynomial active at the same
-// extended limbs, and no output that is also the digits', a key's or another output's polynomial.
+// extended limbs, rows in their block's order, and no output that is also the digits', a key's or
+// another output's polynomial.
 bool gadget_all_ok(RNS_MLWE out, RNS_MLWE* ksk, Poly* poly) {
     IncNtt* t = pool(out);
     const uint64_t ext = ksk[0]->b->rns_mask, mask = poly->pub.rns_mask;
     const int nd = popcount64(mask), comps = (int)out->r + 1;
     if (nd == 0 || comps > kGadgetComps || comps < 2 || nd * comps > kGadgetKeys || t->pub.l > 64) return false;
     auto covers = [&](Poly* p, uint64_t m) {
-        return p && p->base && pool_of(p) == t && (p->pub.allocated_l >= 64 || (m >> p->pub.allocated_l) == 0);
+        if (!p || !p->base || pool_of(p) != t || (p->pub.allocated_l < 64 && (m >> p->pub.allocated_l) != 0)) return false;
+        for (uint64_t rows = m; rows; rows &= rows - 1) {
+            const int i = __builtin_ctzll(rows);
+            if (p->pub.coeffs[i] != p->base + i * t->pub.N) return false;
+        }
+        return true;
     };
     if (!covers(poly, mask) || (t->pub.l < 64 && (ext >> t->pub.l) != 0)) return false;
     uint32_t idx[64];
