@@ -72,7 +72,7 @@ def test_a_class_is_timed_over_its_range():
 
     for b in BUCKETS:
         counts = row_counts(b)
-        assert len(counts) == 3 and all(c >> b == 1 and c % 3 == 0 for c in counts)
+        assert len(counts) in (3, 4) and all(c >> b == 1 and c % 3 == 0 for c in counts)
         assert any(c % 2 for c in counts) and any(c % (1 << (b - 1)) == 0 for c in counts)
         assert counts[-1] > 1.7 * (1 << b)
 

@@ -5,10 +5,15 @@ FP64 transform -- tile bits (one pass, or a radix-2^(logP - tile_bits) column pa
 followed by tiles), tiles per CTA, and one-CTA-per-tile-group vs a persistent grid of
 k CTAs per SM -- on forward + inverse transforms of several row counts of the class (odd
 and even, from its start to its end), and keeps the one whose times, relative to the built-in
-schedule's, have the least mean.  Schedules never change results (the transform is exact), so a tuned table
-can be applied at any time.  The table is a JSON file keyed "logP/rows_log2";
+schedule's, have the least mean.  Schedules never change results (the transform is exact),
+so a tuned table can be applied at any time.  The table is a JSON file keyed "logP/rows_log2";
 ``apply`` loads it into the engine and missing classes use the nearest tuned bucket
 of the same logP.
+
+A transform's schedule also sets what a key switch's fused column pass and division finds to
+do behind it (2^tile_bits columns a polynomial), which is not timed here: few rows of 2^13
+points and more want larger tiles than the transform alone does (one multiply at N = 2^15,
+9 limbs: 88 us on 2^11 and 2^12 tiles, 106 on the tiles this tuner prefers).
 
     python -m vfhe_b200.autotune --out vfhe_b200/tuned/ntt_schedule_b200.json
 """
@@ -64,33 +69,54 @@ def flow_supported(k: int, k1: int) -> bool:
 
 
 def row_counts(bucket: int) -> list[int]:
-    """Row counts a class is timed at, multiples of the three limbs of a timed polynomial: an odd
-    one near its start (tiles that do not fill CTAs evenly), three times a power of two (tiles
-    that do), and one near its end."""
+    """Row counts a class is timed at, multiples of the three limbs of a timed polynomial: odd
+    ones near its start and past its middle (tiles that do not fill CTAs evenly), three times a
+    power of two (tiles that do), and one near its end."""
     n = 1 << bucket
-    polys = ((n + n // 8) // 3 | 1, n // 2, (2 * n - n // 8) // 3)
+    polys = ((n + n // 8) // 3 | 1, n // 2, n // 2 + 1 | 1, (2 * n - n // 8) // 3)
     return sorted({3 * b for b in polys if n <= 3 * b < 2 * n})
 
 
-def _device_ms(call, stream, reps: int) -> float:
-    """Device time of call(), an average over launches that queue behind a wait of the device:
-    one by one, the host's launch rate would hide what a schedule does below some 10 us."""
+def _device_ms(call, captured: bool, reps: int) -> float:
+    """Device time of call(stream) the two ways a program launches, averaged: queued on a stream
+    (behind a wait of the device: one by one, the host's launch rate would hide what a schedule
+    does below some 10 us) and, where it can be, captured in a CUDA graph (queued launches start
+    on a grid of about 2 us, which hides smaller differences)."""
     import torch
 
+    stream = torch.cuda.Stream()
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    best, count = float("inf"), 1
-    for rep in range(reps + 1):
-        torch.cuda._sleep(50_000 * (count + 1))
+
+    def best_of(enqueue, count: int) -> float:
+        best = float("inf")
+        for _ in range(reps):
+            torch.cuda._sleep(50_000 * (count + 1))
+            ev0.record(stream)
+            enqueue()
+            ev1.record(stream)
+            stream.synchronize()
+            best = min(best, ev0.elapsed_time(ev1) / count)
+        return best
+
+    with torch.cuda.stream(stream):
+        call(stream)
         ev0.record(stream)
-        for _ in range(count):
-            call()
+        call(stream)
         ev1.record(stream)
         stream.synchronize()
-        if rep:  # (the first one warms up and sets how many fill half a millisecond)
-            best = min(best, ev0.elapsed_time(ev1) / count)
-        else:
-            count = max(1, min(20, int(0.5 / max(ev0.elapsed_time(ev1), 1e-3))))
-    return best
+        count = max(1, min(20, int(0.5 / max(ev0.elapsed_time(ev1), 1e-3))))
+
+        def several() -> None:
+            for _ in range(count):
+                call(stream)
+
+        queued = best_of(several, count)
+        if not captured:
+            return queued
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            several()
+        return (queued + best_of(graph.replay, count)) / 2
 
 
 def _time_shape(engine: Engine, logP: int, rows: int, cands, reps: int = 5) -> dict[tuple, float]:
@@ -110,12 +136,9 @@ def _time_shape(engine: Engine, logP: int, rows: int, cands, reps: int = 5) -> d
     limbs = ffi.new("uint32_t[]", R.prime_indices)
     p = ffi.cast("uint64_t*", buf.data_ptr())
 
-    st = torch.cuda.current_stream()
-    sp = ffi.cast("void*", st.cuda_stream)
-
-    def both() -> None:
+    def both(stream) -> None:
         for inverse in (0, 1):
-            lib.vfhe_cuda_ntt_batch(R.NTT, inverse, p, p, batch, limbs, L, sp)
+            lib.vfhe_cuda_ntt_batch(R.NTT, inverse, p, p, batch, limbs, L, ffi.cast("void*", stream.cuda_stream))
 
     bucket = (batch * L).bit_length() - 1
     res = {}
@@ -123,7 +146,7 @@ def _time_shape(engine: Engine, logP: int, rows: int, cands, reps: int = 5) -> d
         if lib.vfhe_cuda_ntt_set_schedule(logP, bucket, *c) != 0:
             lib.vfhe_cuda_clear_error()
             continue
-        res[c] = _device_ms(both, st, reps)
+        res[c] = _device_ms(both, c[2] != -2, reps)  # (the dataflow launch does not run under capture)
     lib.vfhe_cuda_ntt_set_schedule(logP, bucket, 0, 0, 0)
     engine.check("autotune")
     return res
