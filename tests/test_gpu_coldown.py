@@ -101,3 +101,46 @@ def test_fused_column_division_matches_unfused_and_single_calls(cuda, N, n_mid, 
     # the rotation with one kernel each
     assert plain[2] - fused[2] == 2
     assert cuda.lib.vfhe_cuda_device_faults() == 0
+
+
+@pytest.mark.parametrize("side", [-1, 0])
+def test_schedules_with_wide_columns_fuse_where_they_fill_the_gpu(cuda, side):
+    """Tiles of 2^8 points leave a 2^13-point row a radix-32 column pass, more than the fused
+    kernel takes; with 512 columns of its own an SM it runs on 2^9 tiles instead."""
+    import torch
+
+    from vfhe_b200.arith import Ring
+    from vfhe_b200.batch import CkksBatch
+
+    n, L = 2**13, 2
+    ring = Ring(n, prime_size=[50, 40, 50], split_degree=1, engine=cuda)
+    batch = CkksBatch(ring.quotient_ring(ell=L), ring.prime_indices[-1])
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    B = -(-512 * sms // (2 << 9)) + side
+
+    def uniform(shape, axis, primes):
+        t = torch.empty(shape, dtype=torch.int64, device="cuda")
+        for k, q in enumerate(primes):
+            t.select(axis, k).random_(0, int(q))
+        return t
+
+    q = list(ring.primes)
+    ct1, ct2 = uniform((B, 2, L, n), 2, q[:L]), uniform((B, 2, L, n), 2, q[:L])
+    key = uniform((L, 2, L + 1, n), 2, q)
+    out, launches = {}, {}
+    with _AllBuckets(cuda.lib, cuda.ffi, 13, (8, 0, 0)):
+        for unfused in (False, True):
+            old = os.environ.pop("VFHE_CUDA_CKKS_UNFUSED", None)
+            if unfused:
+                os.environ["VFHE_CUDA_CKKS_UNFUSED"] = "1"
+            try:
+                n0 = cuda.lib.vfhe_cuda_launch_count()
+                out[unfused] = [batch.mul_relin_rescale(ct1, ct2, key), batch.rotate(ct1, [5] * B, [key] * B)]
+                torch.cuda.synchronize()
+                launches[unfused] = cuda.lib.vfhe_cuda_launch_count() - n0
+            finally:
+                os.environ.pop("VFHE_CUDA_CKKS_UNFUSED", None)
+                if old is not None:
+                    os.environ["VFHE_CUDA_CKKS_UNFUSED"] = old
+    assert all(torch.equal(a, b) for a, b in zip(out[False], out[True]))
+    assert launches[True] - launches[False] == (2 if side == 0 else 0)

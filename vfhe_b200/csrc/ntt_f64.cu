@@ -653,16 +653,27 @@ int launch_ntt_f64(const RowSet& rows, const PrimeInfo* d_primes, bool inverse, 
 }
 
 // The tile pass of an inverse transform whose schedule is a plain tile pass + column
-// pass with at most `max_k1` column bits: the rows are left as centred doubles for a
-// caller that fuses the column pass (and what follows it) into its own kernel.  Returns
-// kTilePassUnavailable, having enqueued nothing, for any other schedule.
+// pass with at most `max_k1` column bits (or is made one, below): the rows are left as centred
+// doubles for a caller that fuses the column pass (and what follows it) into its own kernel.
+// Returns kTilePassUnavailable, having enqueued nothing, for any other schedule.
 int launch_ntt_f64_inverse_tiles(const RowSet& rows, const PrimeInfo* d_primes, int max_k1, int* K1_out, int* KT_out,
                                  cudaStream_t stream) {
     const int logP = rows.logP;
     if (!ntt_f64_eligible(rows)) return kTilePassUnavailable;
-    const NttSchedule sc = get_ntt_schedule(logP, rowset_rows(rows));
+    NttSchedule sc = get_ntt_schedule(logP, rowset_rows(rows));
     int K = sc.tile_bits ? sc.tile_bits : (logP <= 13 ? logP : 12);
     if (K > logP || logP - K > 5) K = logP <= 13 ? logP : 12;
+    // A schedule whose tiles leave the caller too many column bits: larger tiles up to 2^12, where
+    // the caller's kernel (a thread a column, every limb in turn) then fills the GPU, 512 threads
+    // an SM.  Key switches, this schedule with the division on its own and fused on larger tiles:
+    // 40 rotations at N = 2^16, 2 limbs 414 and 385 us, 24 multiplies at 2^15, 9 limbs 893 and 871;
+    // with fewer columns 3 rotations at 2^16, 24 limbs 1426 and 1453, 5 at 2^15, 18 limbs 599 and 642.
+    const int Kc = logP - max_k1;
+    if (K < Kc && Kc <= 12 && sc.ctas_per_sm >= 0 &&
+        ((long long)rows.batch * rows.split << Kc) >= 512LL * sm_count()) {
+        K = Kc;
+        sc = NttSchedule{K, 0, 0};
+    }
     const int K1 = logP - K;
     if (K1 < 1 || K1 > max_k1 || sc.ctas_per_sm < 0) return kTilePassUnavailable;
     *K1_out = K1;
