@@ -60,7 +60,7 @@ __device__ __forceinline__ int lane_tw_index(int g, int b, int h) {
 // How a kernel wants its tiles' addresses and residues: kWhole and kSplit differ in the exchange
 // and twiddle addresses of tiles whose passes all have four stages (see fput_at); kLinear is
 // kSplit with 16 consecutive residues a thread at bit 0, for kernels that keep that pass's
-// residues in shared memory (chain.cu).
+// residues in shared memory (chain.cu) and where a launch is one tile's latency (inverse_form).
 enum TileForm { kWhole, kSplit, kLinear };
 
 // Bits of the layout of a tile's pass at bit 0 (the forward transform's last, the inverse's
